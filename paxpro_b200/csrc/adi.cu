@@ -10,12 +10,12 @@
 // A CTA owns G consecutive systems.  It stages them, plus one halo system on
 // each side for the explicit stencil, in shared memory with loads that are
 // coalesced for either layout (systems interleaved in memory for the x half
-// step, contiguous for the y half step).  Each system is split into
-// P = n/M chunks, one per thread; the chunk rows are built with the
-// reference's operation order (matrix coefficients equal the reference's),
-// the chunk interior is eliminated in registers, and the 2P-unknown reduced
-// system is solved by cyclic reduction in shared memory.  The solution goes
-// back through shared memory for coalesced stores.
+// step, contiguous for the y half step).  Each system is split into chunks,
+// one per thread; the diagonals are built with the reference's operation
+// order (matrix coefficients equal the reference's), the chunk interior is
+// eliminated in registers, and the reduced system, one unknown a chunk, is
+// solved by parallel cyclic reduction.  The solution goes back through shared
+// memory for coalesced stores.
 //
 // Materials: a first-hit sphere list evaluated per point with rounded FP64
 // operations (the same r^2 < R^2 test as the oracle); the host culls, per
@@ -30,7 +30,6 @@
 #include "pxp_complex.cuh"
 #include "pxp_kernels.h"
 #include "scan_solve.cuh"
-#include "tridiag.cuh"
 
 namespace pxp {
 
@@ -79,175 +78,344 @@ __device__ __forceinline__ double2 tbc_factor(double2 num, double2 den) {
   return cx_mul_rn(mk(0.0, 0.5), mk(e * cs, e * sn));
 }
 
-// Diagonal of the padding rows of a system padded to M times a power of two.
+// Diagonal of the rows that pad a system to whole chunks.
 constexpr double kAdiPad = 1e30;
 
-template <typename R, int M, int G>
-__global__ void __launch_bounds__(512) adi_half_kernel(const AdiHalf h) {
+__device__ __forceinline__ void group_sync(int id, int count) {
+  asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(count) : "memory");
+}
+
+// Diagonal of the row at (x, y), from the plane's material there.
+__device__ __forceinline__ double2 adi_diag(const AdiHalf &h, double x, double y, long long idx,
+                                            double inv_impl) {
+  double delta, beta;
+  sphere_material(h, x, y, idx, delta, beta);
+  if (!h.y_implicit)  // 1.0/dz + i/(k dx dx) + beta*k + i*delta*k   (reference :38)
+    return mk(__dadd_rn(h.inv_dzh, __dmul_rn(beta, h.k)), __dadd_rn(inv_impl, __dmul_rn(delta, h.k)));
+  // 1.0/dz + i/(k dy dy + beta*k + i*delta*k)   (reference :103, as written);
+  // in vacuum i/(k dy dy) exactly
+  double2 d = mk(0.0, inv_impl);
+  if (delta != 0.0 || beta != 0.0)
+    d = cx_div_rn(mk(0.0, 1.0),
+                  mk(__dadd_rn(h.kd2_impl, __dmul_rn(beta, h.k)), __dmul_rn(delta, h.k)));
+  return mk(__dadd_rn(d.x, h.inv_dzh), d.y);
+}
+
+// Transparent ends: what the diagonal of a system's end row loses (edge: the
+// field there, inner: beside it), and what the right-hand side of the first
+// and last system gains.  Out of line: few rows reach them.
+__device__ __noinline__ double2 adi_tbc_diag(double2 edge, double2 inner, double kd2) {
+  if (!(hypot(inner.x, inner.y) > 1e-6)) return mk(0.0, 0.0);
+  return cx_div_real_rn(tbc_factor(edge, inner), kd2);
+}
+__device__ __noinline__ double2 adi_tbc_rhs(double2 edge, double2 inner, double kd2) {
+  if (!(hypot(inner.x, inner.y) > 1e-6)) return mk(0.0, 0.0);
+  return cx_div_real_rn(cx_mul_rn(tbc_factor(edge, inner), edge), kd2);
+}
+
+// 1/m for 1e-300 < m < 1e300: the hardware's approximate reciprocal and two
+// Newton steps (error below 2 ulp).  1.0/m adds a branch to a subroutine for
+// other arguments, which the row chain would pay for at every row.
+__device__ __forceinline__ double rcp_newton(double m) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(m));
+  r = fma(r, fma(-m, r, 1.0), r);
+  return fma(r, fma(-m, r, 1.0), r);
+}
+__device__ __forceinline__ double2 crecip_newton(double2 b) {
+  const double r = rcp_newton(fma(b.x, b.x, b.y * b.y));
+  return mk(b.x * r, -b.y * r);
+}
+
+__device__ __forceinline__ double2 shfl_up2(double2 v, int d) {
+  return mk(__shfl_up_sync(0xffffffffu, v.x, d), __shfl_up_sync(0xffffffffu, v.y, d));
+}
+__device__ __forceinline__ double2 shfl_down2(double2 v, int d) {
+  return mk(__shfl_down_sync(0xffffffffu, v.x, d), __shfl_down_sync(0xffffffffu, v.y, d));
+}
+template <int BYTES>
+__device__ __forceinline__ void adi_cp_async(void *dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src), "n"(BYTES)
+               : "memory");
+}
+
+// Shared memory of the general half step: G + 2 staged systems, the diagonals
+// of its G, and the reduction's buffers for more than one warp a system (in
+// the place of the diagonals for the longest systems, whose staging fills
+// shared memory).
+__host__ __device__ constexpr bool adi_own_red(int M, int W) { return W > 1 && M * W < 36; }
+template <typename R, int M, int W, int G> constexpr size_t adi_chunk_smem() {
+  return sizeof(typename Cx<R>::T) * (G + 2) * (32 * W * M) + sizeof(double2) * G * (32 * W * M) +
+         (adi_own_red(M, W) ? sizeof(double2) * G * 8 * 32 * W : 0);
+}
+
+// General half step (planes with material, transparent ends): G systems a
+// CTA, W warps a system, thread c of a system owning rows c*M .. c*M+M-1.
+//
+// With the off-diagonal s on both sides a chunk's rows but the last are
+// eliminated in one forward sweep, x_i + cp_i x_(i+1) = y_i + p_i X_(c-1), X_c
+// the value of chunk c's last row, p_i the running product of -cp; the same
+// sweep accumulates x_0 = Y0 + P0 X_(c-1) + Q0 X_c as Y0 = sum pi_i y_i, P0 =
+// sum pi_i p_i, Q0 = p_(M-2) (pi_i = p_(i-1); the matrix is symmetric).  The
+// last rows then form a symmetric tridiagonal system with one unknown a
+// thread, solved by parallel cyclic reduction -- in registers with shuffles
+// for one warp a system, through double-buffered shared memory and a named
+// barrier a level for more.  Each thread adds its carry-in and substitutes
+// back.  One reciprocal a row and one a reduction level.
+//
+// What bounds it: the latency of the row chain (reciprocal, then the products
+// that wait for it) with few warps an SM, about 10 cycles an instruction and
+// warp; FP64 issue is about 56 operations a point (19 % of the pipe at 513
+// nodes).  So a system is spread over several warps with short chunks, and
+// the diagonals -- the only part that needs the material lookups, divisions
+// and branches -- are formed for the whole CTA in staging order before the
+// unrolled sweep, while the field's copies arrive.  Inlined into the sweep
+// they outgrow the instruction cache (21 against 14 us a half step at 513).
+//
+// Measured, whole steps of a sphere that fills the domain (FP64, us a step,
+// before: chunks of 8 rows, two unknowns a chunk, cyclic reduction over the
+// CTA with a barrier a level, systems padded to 8 * 2^k): 150 nodes 43.4 ->
+// 11.1, 256: 42.1 -> 12.7, 600: 98 -> 31.6, 700: 101 -> 39.3, 1024: 108 ->
+// 56.3, 1500: 407 -> 144; 513 over 64 steps, 20 of them vacuum, 58.4 -> 21.1.
+template <typename R, int M, int W, int G, bool TBC>
+__global__ void __launch_bounds__(32 * W *G) adi_chunk_kernel(const __grid_constant__ AdiHalf h) {
   using C = typename Cx<R>::T;
+  constexpr int P = 32 * W, T = P * G, LD = P * M, RW = G + 2;
+  static_assert(M % 2 == 1, "an odd chunk stride: a warp's lanes hit different bank groups");
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  // n: rows of each solved system (h.n, or h.n padded to M times a power of
-  // two); nreal: the grid's positions per system and its number of systems.
-  // Pad rows get diagonal kAdiPad, zero right-hand side and zero field, so
-  // they decouple from the last real row to within |sub|^2 / kAdiPad.
-  const int n = h.n_pad > 0 ? h.n_pad : h.n;
-  const int nreal = h.n;
-  const int P = n / M;        // chunks per system
-  const int T = G * P;        // threads
-  const int ld = n + n / 8 + 2;  // padded row of the staging tile (pad8)
-  C *tile = reinterpret_cast<C *>(smem_raw);                  // (G+2) x ld
-  double2 *red = reinterpret_cast<double2 *>(
-      smem_raw + ((sizeof(C) * (G + 2) * ld + 15) & ~size_t(15)));  // 4 x G x 2P
-  const int nr = 2 * P;
+  double2 *diag = reinterpret_cast<double2 *>(smem_raw);  // G x LD
+  constexpr bool OWN_RED = adi_own_red(M, W);
+  C *tile = reinterpret_cast<C *>(diag + G * LD + (OWN_RED ? G * 8 * P : 0));  // RW x LD
+  const int n = h.n;
   const int tid = threadIdx.x;
-  const int s_base = blockIdx.x * G;  // first system of this CTA
+  const int s_base = blockIdx.x * G;
   const C *in = reinterpret_cast<const C *>(h.in);
   C *out = reinterpret_cast<C *>(h.out);
   const bool interleaved = h.stride_sys == 1;
+  const int nsys = n - s_base < G ? n - s_base : G;  // the last CTA may hold fewer
+  constexpr int PPI = T / RW;  // x half step: positions staged at a time
+  constexpr int PPO = T / G;   // and stored
 
-  // ---- stage systems s_base-1 .. s_base+G (out-of-range halo rows zero)
-  const int rows = G + 2;
-  for (int idx = tid; idx < rows * n; idx += T) {
-    int g, p;
-    if (interleaved) {
-      p = idx / rows;
-      g = idx - p * rows;
-    } else {
-      g = idx / n;
-      p = idx - g * n;
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  // ---- stage systems s_base-1 .. s_base+G; outside the grid the field is zero
+  if (interleaved) {
+    // adjacent systems are adjacent in memory: consecutive threads take them
+    const int g = tid % RW, sys = s_base - 1 + g;
+    if (tid < PPI * RW) {
+      C *dst = tile + g * LD;
+      if (sys >= 0 && sys < n)
+        for (int p = tid / RW; p < n; p += PPI)
+          adi_cp_async<sizeof(C)>(dst + p, in + (long long)p * h.stride_pos + sys);
+      else
+        for (int p = tid / RW; p < n; p += PPI) dst[p] = C{};
     }
-    const int s = s_base - 1 + g;
-    C v = from_d<R>(mk(0.0, 0.0));
-    if (s >= 0 && s < nreal && p < nreal)
-      v = in[(long long)p * h.stride_pos + (long long)s * h.stride_sys];
-    tile[g * ld + pad8(p)] = v;
+  } else {
+    for (int g = 0; g < RW; ++g) {
+      const int sys = s_base - 1 + g;
+      const C *src = in + (long long)sys * h.stride_sys;
+      C *dst = tile + g * LD;
+      if (sys >= 0 && sys < n)
+        for (int p = tid; p < n; p += T) adi_cp_async<sizeof(C)>(dst + p, src + p);
+      else
+        for (int p = tid; p < n; p += T) dst[p] = C{};
+    }
   }
+  const double q = __ddiv_rn(0.5, h.kd2_impl);  // the off-diagonal is -i q
+  const double inv_impl = __ddiv_rn(1.0, h.kd2_impl);
+  const double inv_expl = __ddiv_rn(1.0, h.kd2_expl);
+  const double hk = 0.5 * inv_expl;
+  // ---- diagonals, while the field arrives
+  if (interleaved) {
+    const int gg = tid % G, sys = s_base + gg;
+    const double y = __dadd_rn(h.ymin, __dmul_rn((double)sys, h.dy));
+    if (tid < PPO * G)
+      for (int p = tid / G; p < LD; p += PPO) {
+        const double x = __dadd_rn(h.xmin, __dmul_rn((double)p, h.dx));
+        diag[gg * LD + p] = p < n && gg < nsys ? adi_diag(h, x, y, (long long)p * n + sys, inv_impl)
+                                               : mk(kAdiPad, 0.0);
+      }
+  } else {
+#pragma unroll 1
+    for (int gg = 0; gg < G; ++gg) {
+      const int sys = s_base + gg;
+      const double x = __dadd_rn(h.xmin, __dmul_rn((double)sys, h.dx));
+      for (int p = tid; p < LD; p += T) {
+        const double y = __dadd_rn(h.ymin, __dmul_rn((double)p, h.dy));
+        diag[gg * LD + p] = p < n && gg < nsys ? adi_diag(h, x, y, (long long)sys * n + p, inv_impl)
+                                               : mk(kAdiPad, 0.0);
+      }
+    }
+  }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
   __syncthreads();
 
-  const int g = tid / P;          // system within the CTA
-  const int c = tid - g * P;      // chunk
-  const int s = s_base + g;       // global system index
+  const int g = tid / P, c = tid % P;
+  const int s = s_base + g;
   const int p0 = c * M;
-  const double2 sub = mk(-0.0, __ddiv_rn(-0.5, h.kd2_impl));  // -0.5*i/(k d^2)
-  const double inv_kd2_impl = __ddiv_rn(1.0, h.kd2_impl);
-  const double inv_kd2_expl = __ddiv_rn(1.0, h.kd2_expl);
-  // y half step diagonal in vacuum: i/(k dy^2 + 0 + i 0) = (0, 1/(k dy^2))
-  // exactly (Smith's division with a zero imaginary part).
-  const C *ctr = tile + (g + 1) * ld;
-  const C *lft = tile + g * ld;
-  const C *rgt = tile + (g + 2) * ld;
-
-  double2 dg[M], rh[M];
-#pragma unroll
-  for (int m = 0; m < M; ++m) {
-    const int p = p0 + m;
-    if (p >= nreal) {
-      dg[m] = mk(kAdiPad, 0.0);
-      rh[m] = mk(0.0, 0.0);
-      continue;
-    }
-    // coordinates: position runs along x in the x half step, along y in the y half step
-    double x, y;
-    const double pos_c = (double)p, sys_c = (double)s;
-    if (!h.y_implicit) {
-      x = __dadd_rn(h.xmin, __dmul_rn(pos_c, h.dx));
-      y = __dadd_rn(h.ymin, __dmul_rn(sys_c, h.dy));
-    } else {
-      x = __dadd_rn(h.xmin, __dmul_rn(sys_c, h.dx));
-      y = __dadd_rn(h.ymin, __dmul_rn(pos_c, h.dy));
-    }
-    double delta, beta;
-    sphere_material(h, x, y,
-                    h.y_implicit ? (long long)s * h.n + p : (long long)p * h.n + s, delta, beta);
-    if (!h.y_implicit) {
-      // 1.0/dz + i/(k dx dx) + beta*k + i*delta*k   (reference :38)
-      dg[m] = mk(__dadd_rn(h.inv_dzh, __dmul_rn(beta, h.k)),
-                 __dadd_rn(inv_kd2_impl, __dmul_rn(delta, h.k)));
-    } else {
-      // 1.0/dz + i/(k dy dy + beta*k + i*delta*k)   (reference :103, as written)
-      double2 q = mk(0.0, inv_kd2_impl);
-      if (delta != 0.0 || beta != 0.0)
-        q = cx_div_rn(mk(0.0, 1.0), mk(__dadd_rn(h.kd2_impl, __dmul_rn(beta, h.k)),
-                                       __dmul_rn(delta, h.k)));
-      dg[m] = mk(__dadd_rn(q.x, h.inv_dzh), q.y);
-    }
-    // rhs = (1/dz - i/(k d_e^2)) u + 0.5 i (u_left + u_right)/(k d_e^2); the
-    // reference divides each neighbour term by k d_e^2, here it is one
-    // multiplication by the reciprocal (a rounding-level difference).
-    const double2 uc = to_d(ctr[pad8(p)]);
-    double2 r = cmul(mk(h.inv_dzh, -inv_kd2_expl), uc);
-    double2 nb = mk(0.0, 0.0);
-    if (s > 0) nb = to_d(lft[pad8(p)]);
-    if (s < nreal - 1) nb = cadd(nb, to_d(rgt[pad8(p)]));
-    const double hk = 0.5 * inv_kd2_expl;
-    r = mk(fma(-hk, nb.y, r.x), fma(hk, nb.x, r.y));
-    rh[m] = r;
-  }
-  if (h.use_tbc) {
-    const double zero = 1e-6;
-    // along the system (implicit direction): diagonal at both ends (the last
-    // real row: row n - 1 of an unpadded system)
-    if (p0 <= nreal - 1 && nreal - 1 < p0 + M) {
-      double2 inner = to_d(ctr[pad8(nreal - 2)]);
-      if (hypot(inner.x, inner.y) > zero) {
-        const double2 t = cx_div_real_rn(tbc_factor(to_d(ctr[pad8(nreal - 1)]), inner), h.kd2_impl);
-#pragma unroll
-        for (int m = 0; m < M; ++m)
-          if (p0 + m == nreal - 1) dg[m] = cx_sub_rn(dg[m], t);
-      }
-    }
-    if (c == 0) {
-      double2 inner = to_d(ctr[pad8(1)]);
-      if (hypot(inner.x, inner.y) > zero)
-        dg[0] = cx_sub_rn(dg[0], cx_div_real_rn(tbc_factor(to_d(ctr[pad8(0)]), inner), h.kd2_impl));
-    }
-    // across systems (explicit direction): rhs of the first and last system
-    if (s == nreal - 1 || s == 0) {
-      const C *inner_row = (s == nreal - 1) ? lft : rgt;
-#pragma unroll
-      for (int m = 0; m < M; ++m) {
-        const int p = p0 + m;
-        if (p >= nreal) continue;
-        double2 inner = to_d(inner_row[pad8(p)]);
-        if (hypot(inner.x, inner.y) > zero) {
-          double2 edge = to_d(ctr[pad8(p)]);
-          double2 f = cx_mul_rn(tbc_factor(edge, inner), edge);
-          rh[m] = cx_add_rn(rh[m], cx_div_real_rn(f, h.kd2_expl));
-        }
-      }
-    }
+  const C *ctr = tile + (g + 1) * LD + p0;
+  const C *lft = ctr - LD, *rgt = ctr + LD;
+  double2 *dgs = diag + g * LD + p0;
+  auto smul = [q](double2 z) { return mk(q * z.y, -q * z.x); };  // off-diagonal * z
+  if (TBC && g < nsys) {
+    // the diagonal of the system's two end rows
+    const C *sysv = tile + (g + 1) * LD;
+    if (c == 0) dgs[0] = cx_sub_rn(dgs[0], adi_tbc_diag(to_d(sysv[0]), to_d(sysv[1]), h.kd2_impl));
+    if (p0 <= n - 1 && n - 1 < p0 + M)
+      dgs[n - 1 - p0] = cx_sub_rn(
+          dgs[n - 1 - p0], adi_tbc_diag(to_d(sysv[n - 1]), to_d(sysv[n - 2]), h.kd2_impl));
   }
 
-  double2 yv[M > 2 ? M - 2 : 1], pv[M > 2 ? M - 2 : 1], qv[M > 2 ? M - 2 : 1];
-  const ReducedRows rr = chunk_eliminate<M>(dg, rh, sub, p0 > 0, p0 + M < n, yv, pv, qv);
-  double2 *ra = red + (0 * G + g) * nr;
-  double2 *rb = red + (1 * G + g) * nr;
-  double2 *rc = red + (2 * G + g) * nr;
-  double2 *rd = red + (3 * G + g) * nr;
-  ra[2 * c] = rr.ea; rb[2 * c] = rr.eb; rc[2 * c] = rr.ec; rd[2 * c] = rr.ed;
-  ra[2 * c + 1] = rr.fa; rb[2 * c + 1] = rr.fb; rc[2 * c + 1] = rr.fc; rd[2 * c + 1] = rr.fd;
-  __syncthreads();  // also: every read of the staged tile is done
-  cyclic_reduction(ra, rb, rc, rd, nr, c, P);
-  const double2 xf = rd[2 * c], xl = rd[2 * c + 1];
-  C *dst = tile + (g + 1) * ld;
+  // diagonal and right-hand side of row m (position p0 + m) of this chunk
+  auto row = [&](int m, double2 &dg, double2 &rh) {
+    dg = dgs[m];
+    rh = mk(0.0, 0.0);
+    if (p0 + m >= n || g >= nsys) return;
+    // (1/dz - i/(k d_e^2)) u + 0.5 i (u_left + u_right)/(k d_e^2)
+    const double2 r = cmul(mk(h.inv_dzh, -inv_expl), to_d(ctr[m]));
+    const double2 nb = cadd(to_d(lft[m]), to_d(rgt[m]));
+    rh = mk(fma(-hk, nb.y, r.x), fma(hk, nb.x, r.y));
+    if (TBC && (s == 0 || s == n - 1))
+      rh = cx_add_rn(rh, adi_tbc_rhs(to_d(ctr[m]), to_d(s == n - 1 ? lft[m] : rgt[m]), h.kd2_expl));
+  };
+
+  // ---- forward sweep over rows 0 .. M-2
+  double2 cp[M - 1], yv[M - 1];
+  double2 pi = mk(1.0, 0.0), y0 = mk(0.0, 0.0), pp0 = mk(0.0, 0.0);
 #pragma unroll
-  for (int m = 0; m < M; ++m) dst[pad8(p0 + m)] = from_d<R>(chunk_value<M>(m, xf, xl, yv, pv, qv));
+  for (int m = 0; m < M - 1; ++m) {
+    double2 dg, rh;
+    row(m, dg, rh);
+    if (m > 0) {
+      dg = csub(dg, smul(cp[m - 1]));
+      rh = csub(rh, smul(yv[m - 1]));
+    }
+    const double2 inv = crecip_newton(dg);
+    cp[m] = smul(inv);
+    yv[m] = cmul(rh, inv);
+    y0 = cfma(pi, yv[m], y0);
+    const double2 t = cmul(cp[m], pi);
+    const double2 pn = mk(-t.x, -t.y);
+    pp0 = cfma(pi, pn, pp0);
+    pi = pn;
+  }
+  // ---- the last row's equation a X_(c-1) + b X_c + e X_(c+1) = d
+  double2 b, d;
+  row(M - 1, b, d);
+  b = csub(b, smul(cp[M - 2]));
+  d = csub(d, smul(yv[M - 2]));
+  double2 a = c > 0 ? smul(pi) : mk(0.0, 0.0);
+  double2 e = mk(0.0, 0.0);
+  double2 x, xl;
+  if constexpr (W == 1) {
+    const double2 ry = shfl_down2(y0, 1), rp = shfl_down2(pp0, 1), rq = shfl_down2(pi, 1);
+    if (c < P - 1) {
+      b = cadd(b, smul(rp));
+      d = csub(d, smul(ry));
+      e = smul(rq);
+    }
+#pragma unroll
+    for (int sh = 1; sh < P; sh <<= 1) {
+      const double2 r = crecip_newton(b);
+      const double2 dn = cmul(d, r), an = cmul(a, r), en = cmul(e, r);
+      const double2 rl = shfl_up2(r, sh), dl = shfl_up2(dn, sh), al = shfl_up2(an, sh);
+      const double2 rr = shfl_down2(r, sh), dr = shfl_down2(dn, sh), er = shfl_down2(en, sh);
+      // lanes without a neighbour at this distance hold a = 0 (e = 0)
+      b = csub(b, cadd(cmul(a, cmul(a, rl)), cmul(e, cmul(e, rr))));
+      d = csub(d, cadd(cmul(a, dl), cmul(e, dr)));
+      const double2 a2 = cmul(a, al), e2 = cmul(e, er);
+      a = mk(-a2.x, -a2.y);
+      e = mk(-e2.x, -e2.y);
+    }
+    x = cmul(d, crecip_newton(b));
+    xl = shfl_up2(x, 1);
+  } else {
+    // two alternating buffers of P x {reciprocal, d, a, e}: a thread writes
+    // a buffer again only after the barrier that follows every read of it
+    double2 *buf = OWN_RED ? diag + G * LD + g * 8 * P : diag + g * LD;
+    if (!OWN_RED) group_sync(1 + g, P);  // the system's diagonals are read
+    buf[c] = y0;
+    buf[P + c] = pp0;
+    buf[2 * P + c] = pi;
+    group_sync(1 + g, P);
+    if (c < P - 1) {
+      b = cadd(b, smul(buf[P + c + 1]));
+      d = csub(d, smul(buf[c + 1]));
+      e = smul(buf[2 * P + c + 1]);
+    }
+    int k = 1;
+#pragma unroll 1
+    for (int sh = 1; sh < P; sh <<= 1, k ^= 1) {
+      double2 *w = buf + k * 4 * P;
+      const double2 r = crecip_newton(b);
+      w[c] = r;
+      w[P + c] = cmul(d, r);
+      w[2 * P + c] = cmul(a, r);
+      w[3 * P + c] = cmul(e, r);
+      group_sync(1 + g, P);
+      double2 nb = b, nd = d, na = mk(0.0, 0.0), ne = mk(0.0, 0.0);
+      if (c >= sh) {
+        const int j = c - sh;
+        nb = csub(nb, cmul(a, cmul(a, w[j])));
+        nd = csub(nd, cmul(a, w[P + j]));
+        na = cmul(a, w[2 * P + j]);
+      }
+      if (c + sh < P) {
+        const int j = c + sh;
+        nb = csub(nb, cmul(e, cmul(e, w[j])));
+        nd = csub(nd, cmul(e, w[P + j]));
+        ne = cmul(e, w[3 * P + j]);
+      }
+      b = nb;
+      d = nd;
+      a = mk(-na.x, -na.y);
+      e = mk(-ne.x, -ne.y);
+    }
+    x = cmul(d, crecip_newton(b));
+    buf[k * 4 * P + c] = x;
+    group_sync(1 + g, P);
+    xl = c > 0 ? buf[k * 4 * P + c - 1] : mk(0.0, 0.0);
+  }
+  // ---- carry-in, then back substitution; results through the tile
+  if (c > 0) {
+    double2 t = xl;
+#pragma unroll
+    for (int m = 0; m < M - 1; ++m) {
+      t = cmul(cp[m], t);
+      t = mk(-t.x, -t.y);
+      yv[m] = cadd(yv[m], t);
+    }
+  }
+  __syncthreads();  // every read of the staged systems is done
+  C *dst = tile + (g + 1) * LD + p0;
+  dst[M - 1] = from_d<R>(x);
+#pragma unroll
+  for (int m = M - 2; m >= 0; --m) {
+    x = csub(yv[m], cmul(cp[m], x));
+    dst[m] = from_d<R>(x);
+  }
   __syncthreads();
   C *save = reinterpret_cast<C *>(h.save);
-  for (int idx = tid; idx < G * n; idx += T) {
-    int gg, p;
-    if (interleaved) {
-      p = idx / G;
-      gg = idx - p * G;
-    } else {
-      gg = idx / n;
-      p = idx - gg * n;
+  if (interleaved) {
+    const int gg = tid % G;
+    if (tid < PPO * G && gg < nsys)
+      for (int p = tid / G; p < n; p += PPO) {
+        const long long off = (long long)p * h.stride_pos + s_base + gg;
+        const C v = tile[(gg + 1) * LD + p];
+        out[off] = v;
+        if (save) save[off] = v;
+      }
+  } else {
+    for (int gg = 0; gg < nsys; ++gg) {
+      const long long base = (long long)(s_base + gg) * h.stride_sys;
+      for (int p = tid; p < n; p += T) {
+        const C v = tile[(gg + 1) * LD + p];
+        out[base + p] = v;
+        if (save) save[base + p] = v;
+      }
     }
-    if (p >= nreal || s_base + gg >= nreal) continue;
-    const long long off = (long long)p * h.stride_pos + (long long)(s_base + gg) * h.stride_sys;
-    const C v = tile[(gg + 1) * ld + pad8(p)];
-    out[off] = v;
-    if (save) save[off] = v;
   }
 }
 
@@ -394,10 +562,6 @@ __device__ __forceinline__ void adi_cp_async16(void *smem, const void *gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
 }
 
-
-__device__ __forceinline__ void group_sync(int id, int count) {
-  asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(count) : "memory");
-}
 
 template <bool DOWN>
 __device__ __forceinline__ double2 shfl2(double2 v, int d) {
@@ -1009,51 +1173,59 @@ cudaError_t launch_adi_half_const(Precision p, const AdiHalf &h, const void *g, 
 #undef PXP_AC
 }
 
-static constexpr int kAdiM = 8;
-
-template <int G> constexpr int adi_threads(int n) { return G * (n / kAdiM); }
-
-template <typename R, int G>
-static cudaError_t adi_launch_g(const AdiHalf &h, cudaStream_t s) {
-  using C = typename Cx<R>::T;
-  const int n = h.n_pad > 0 ? h.n_pad : h.n;  // solved system length
-  const int T = adi_threads<G>(n);
-  const size_t tile = (sizeof(C) * (G + 2) * (n + n / 8 + 2) + 15) & ~size_t(15);
-  const size_t smem = tile + sizeof(double2) * 4 * G * 2 * (n / kAdiM);
-  auto k = adi_half_kernel<R, kAdiM, G>;
-  // raise the dynamic shared-memory limit on this device to the largest size
-  // the instantiation can need (n = 2048 for G = 2, n = 1024 for G = 4)
-  const cudaError_t attr = raise_dynamic_smem(
-      (const void *)k,
-      (int)(((sizeof(C) * (G + 2) * (G == 2 ? 2048 + 258 : 1024 + 130) + 15) & ~size_t(15)) +
-            sizeof(double2) * 4 * G * 2 * ((G == 2 ? 2048 : 1024) / kAdiM)));
+template <typename R, int M, int W, int G>
+static cudaError_t adi_chunk_launch_t(const AdiHalf &h, cudaStream_t s) {
+  constexpr size_t smem = adi_chunk_smem<R, M, W, G>();
+  static_assert(smem <= 227 * 1024, "staged systems exceed shared memory");
+  static_assert(W == 1 || G <= 15, "one named barrier per system");
+  auto k = h.use_tbc ? adi_chunk_kernel<R, M, W, G, true> : adi_chunk_kernel<R, M, W, G, false>;
+  const cudaError_t attr = raise_dynamic_smem((const void *)k, (int)smem);
   if (attr != cudaSuccess) return attr;
-  k<<<(h.n + G - 1) / G, T, smem, s>>>(h);  // one CTA per G of the grid's h.n systems
-  return cudaGetLastError();
+  // a programmatic dependent of the previous kernel in the stream: its CTAs
+  // start while that kernel drains and wait for it with griddepcontrol.wait
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((h.n + G - 1) / G);
+  cfg.blockDim = dim3(32 * W * G);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute la[1];
+  la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  la[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = la;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, h);
 }
 
-bool adi_supported(Precision p, int n) {
-  if (n < 64 || (n & (n - 1))) return false;
-  return p == kFP64 ? n <= 2048 : n <= 2048;
-}
+bool adi_size_supported(int n) { return n >= 4 && n <= 2048; }
 
-int adi_padded_n(int n) {
-  if (n >= 64 && !(n & (n - 1))) return n;
-  int t = 8;
-  while (t * kAdiM < n) t *= 2;
-  return t * kAdiM;
-}
+bool adi_supported(Precision, int n) { return n >= 64 && n <= 2048 && !(n & (n - 1)); }
 
-bool adi_padded_supported(Precision p, int n) {
-  return n >= 4 && adi_supported(p, adi_padded_n(n));
+// Rows a thread, warps a system and systems a CTA per grid size.  Two CTAs an
+// SM beat one larger CTA (513: G = 2 21.1 us a step, G = 4 22.8) except where
+// G = 3 still gives at most one CTA an SM (400: 17.1 against 19.2 with G = 2);
+// above 148 CTAs G = 3 leaves SMs with one and SMs with two (513: 31).
+// Complex64 tiles are half as large, and fewer, larger CTAs win (513: G = 4
+// 22.6, G = 2 27.8; 1024: 17 rows and 2 warps 59.9, 9 rows and 4 warps 64.7).
+template <typename R>
+static cudaError_t adi_chunk_launch(const AdiHalf &h, cudaStream_t s) {
+  const int n = h.n;
+  constexpr bool F = sizeof(R) == 4;
+  if (n <= 192) return adi_chunk_launch_t<R, 3, 2, 1>(h, s);
+  if (n <= 384) return adi_chunk_launch_t<R, 3, 4, 2>(h, s);
+  if (n <= 444) return adi_chunk_launch_t<R, 5, 4, 3>(h, s);
+  if (n <= 640) return adi_chunk_launch_t<R, 5, 4, F ? 4 : 2>(h, s);
+  if (n <= 832) return adi_chunk_launch_t<R, 13, 2, F ? 4 : 2>(h, s);
+  if (n <= 1088) {
+    if constexpr (F) return adi_chunk_launch_t<R, 17, 2, 4>(h, s);
+    else return adi_chunk_launch_t<R, 9, 4, 2>(h, s);
+  }
+  if (n <= 1664) return adi_chunk_launch_t<R, 13, 4, 2>(h, s);
+  return adi_chunk_launch_t<R, 17, 4, 1>(h, s);
 }
 
 cudaError_t launch_adi_half(Precision p, const AdiHalf &h, cudaStream_t s) {
-  const int np = h.n_pad > 0 ? h.n_pad : h.n;
-  if (!adi_supported(p, np) || h.n > np) return cudaErrorInvalidValue;
-  // G systems per CTA so that G * n/8 <= 512 threads
-  if (np <= 1024) return p == kFP64 ? adi_launch_g<double, 4>(h, s) : adi_launch_g<float, 4>(h, s);
-  return p == kFP64 ? adi_launch_g<double, 2>(h, s) : adi_launch_g<float, 2>(h, s);
+  if (!adi_size_supported(h.n)) return cudaErrorInvalidValue;
+  return p == kFP64 ? adi_chunk_launch<double>(h, s) : adi_chunk_launch<float>(h, s);
 }
 
 }  // namespace pxp

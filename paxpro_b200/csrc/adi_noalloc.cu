@@ -108,9 +108,6 @@ int run_steps(const pxp_problem *p, pxp::Precision prec, unsigned n, const pxp_s
   const double kdx2 = k * p->x.step * p->x.step, kdy2 = k * p->y.step * p->y.step;
   pxp::AdiHalf a{};
   a.n = (int)n;
-  // sizes other than powers of two: systems padded with decoupled rows, as
-  // the solver handle runs them
-  a.n_pad = pxp::adi_padded_n((int)n) != (int)n ? pxp::adi_padded_n((int)n) : 0;
   a.use_tbc = p->transparent_bc ? 1 : 0;
   a.inv_dzh = 1.0 / dzh;
   a.k = k;
@@ -177,7 +174,7 @@ int pxp_adi_steps_noalloc(const pxp_problem *p, const pxp_sphere *spheres, int n
                   n, n, bytes, kNoAllocScratchBytes);
     return fail(PXP_ERR_UNSUPPORTED, m);
   }
-  if (!pxp::adi_padded_supported(prec, (int)n))
+  if (!pxp::adi_size_supported((int)n))
     return fail(PXP_ERR_UNSUPPORTED, "pxp_adi_steps_noalloc: grid size not supported");
 
   const double dzh = p->z.step / 2.0;  // ADI::xImplicit (src/alternatingDirectionSolver.cpp:18)

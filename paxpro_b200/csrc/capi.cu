@@ -808,7 +808,6 @@ int adi_step(pxp_solver_s *h, unsigned step) {
   const long long n = h->nx;
   pxp::AdiHalf a{};
   a.n = (int)n;
-  a.n_pad = pxp::adi_padded_n((int)n) != (int)n ? pxp::adi_padded_n((int)n) : 0;
   a.use_tbc = p.transparent_bc ? 1 : 0;
   a.inv_dzh = 1.0 / dzh;
   a.k = k;
@@ -1427,9 +1426,7 @@ int pxp_solver_create(const pxp_problem *problem, pxp_solver *out) {
                   (!p.transparent_bc || pxp::cn_padded_n((int)h->nx) == (int)h->nx);
       break;
     case PXP_ADI:
-      // other sizes run padded on the general kernel
-      supported = pxp::adi_supported(h->prec, (int)h->nx) ||
-                  pxp::adi_padded_supported(h->prec, (int)h->nx);
+      supported = pxp::adi_size_supported((int)h->nx);
       break;
     case PXP_FFT_SOLVER_3D: supported = pxp::fft3d_supported(h->prec, (int)h->nx); break;
     default: supported = false;
