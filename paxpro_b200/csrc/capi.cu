@@ -277,7 +277,8 @@ int alloc(pxp_solver_s *h, void **p, size_t bytes, const char *what) {
 struct TableKey {
   int device, kind;  // kind 0: twiddles (radix 8), 1: 1-D propagator, 2: kx^2 per
                      // column, 3: twiddles (radix 16), 4: exp(-2 pi i m / n), m < n,
-                     // 11: the FFTSolver3D register-line kernel's twiddle table
+                     // 11: the FFTSolver3D register-line kernel's twiddle table,
+                     // 12: twiddles of the mixed-radix transform in pass order
   unsigned n;
   double dx, dz, k;
   int split;  // 1: the FP32 split form (split_table), 0: complex128 / doubles
@@ -354,6 +355,28 @@ int shared_table_n(pxp_solver_s *h, int kind, unsigned n, void **out) {
     for (int i = 0; i < cnt; ++i) {
       const long double a = -2.0L * pi_l * (long double)ex[i] / (long double)n;
       t[i] = cd((double)cosl(a), (double)sinl(a));
+    }
+  } else if (kind == 12) {
+    // pass by pass exp(-2 pi i r k / (ns radix)) at (r - 1) * ns + k
+    pxp::MixedPlan plan;
+    if (!pxp::mixed_plan((int)n, &plan)) return h->fail(PXP_ERR_INVALID, "mixed-radix length");
+    const long double pi_l = 3.141592653589793238462643383279502884L;
+    t.reserve(plan.table);
+    for (int p = 0, ns = 1; p < plan.passes; ns *= plan.pass[p].radix, ++p)
+      for (int r = 1; r < plan.pass[p].radix; ++r)
+        for (int k = 0; k < ns; ++k) {
+          const long double a = -2.0L * pi_l * (long double)(r * k) / (long double)(ns * plan.pass[p].radix);
+          t.push_back(cd((double)cosl(a), (double)sinl(a)));
+        }
+    // then (cos, sin)(2 pi j k / radix), j, k = 1 .. radix / 2, of the radices above 9
+    for (int p = 0; p < plan.passes; ++p) {
+      const int r = plan.pass[p].radix, half = r / 2;
+      if (r <= 9 || plan.pass[p].rot != (int)t.size()) continue;
+      for (int k = 1; k <= half; ++k)
+        for (int j = 1; j <= half; ++j) {
+          const long double a = 2.0L * pi_l * (long double)(j * k % r) / (long double)r;
+          t.push_back(cd((double)cosl(a), (double)sinl(a)));
+        }
     }
   } else if (kind == 1) {
     t.resize(n);
@@ -473,9 +496,11 @@ int bluestein_table(pxp_solver_s *h, int kind, void **out) {
 int fft1d_setup(pxp_solver_s *h) {
   int rc;
   if ((rc = shared_table(h, 1, &h->d_kern))) return rc;
-  if (h->nx & (h->nx - 1)) {
-    // not a power of two: the Bluestein path's tables (the Stockham twiddles
-    // are those of its power-of-two length)
+  if (pxp::mixed_plan((int)h->nx, nullptr)) {
+    if ((rc = shared_table(h, 12, &h->d_tw))) return rc;
+  } else if (h->nx & (h->nx - 1)) {
+    // a prime factor above 31: the Bluestein path's tables (the Stockham
+    // twiddles are those of its power-of-two length)
     if ((rc = bluestein_table(h, 7, &h->d_chirp))) return rc;
     if ((rc = bluestein_table(h, 8, &h->d_bconv))) return rc;
     if ((rc = bluestein_table(h, 9, &h->d_tw))) return rc;
@@ -949,7 +974,7 @@ int fft3d_variant(pxp_solver_s *h, const pxp::Fft3dPass &q0, const void *kx2, co
       return PXP_OK;
     }
   }
-  if (h->nx & (h->nx - 1)) {  // one kernel (Bluestein) for other sizes: nothing to tune
+  if (h->nx & (h->nx - 1)) {  // one kernel for other sizes: nothing to tune
     *out = 0;
     return PXP_OK;
   }
@@ -1205,6 +1230,7 @@ int fft3d_steps(pxp_solver_s *h, unsigned first, int nsteps) {
   q.ymin = p.y.min;
   q.dy = p.y.step;
   q.norm = (double)((unsigned)n * (unsigned)n);
+  q.inv_norm = 1.0 / q.norm;
   if (p.absorber_damping > 0.0) {  // FFTSolver3D::absorbingBC (src/fftSolver3D.cpp:327-349)
     q.thick_x = (int)(unsigned)(p.absorber_width / p.x.step + 1);
     q.thick_y = (int)(unsigned)(p.absorber_width / p.y.step + 1);
@@ -1488,8 +1514,10 @@ int pxp_solver_create(const pxp_problem *problem, pxp_solver *out) {
         if ((rc = adi_build_lu(h))) return cleanup_fail(rc);
       break;
     case PXP_FFT_SOLVER_3D:
-      if (h->nx & (h->nx - 1)) {
-        // not a power of two: the Bluestein tables of the line transforms
+      if (pxp::mixed_plan((int)h->nx, nullptr)) {
+        if ((rc = shared_table(h, 12, &h->d_tw))) return cleanup_fail(rc);
+      } else if (h->nx & (h->nx - 1)) {
+        // a prime factor above 31: the Bluestein tables of the line transforms
         if ((rc = bluestein_table(h, 7, &h->d_chirp))) return cleanup_fail(rc);
         if ((rc = bluestein_table(h, 8, &h->d_bconv))) return cleanup_fail(rc);
         if ((rc = bluestein_table(h, 9, &h->d_tw))) return cleanup_fail(rc);

@@ -231,6 +231,8 @@ int fft1d_variants(Precision p, int n) {
 cudaError_t launch_fft1d(Precision p, const Fft1dJob *d_jobs, int nj, int n, int step0,
                          int nsteps, cudaStream_t s, bool flux, int variant, unsigned *queue) {
   if (nj <= 0) return cudaSuccess;
+  if (mixed_plan(n, nullptr))
+    return launch_fft1d_mixed(p, d_jobs, nj, n, step0, nsteps, s, flux);
   if (n & (n - 1)) return launch_bluestein(p, d_jobs, nj, n, step0, nsteps, s, flux);
   if (fft1d_pair_size(p, n)) return launch_fft1d_pair(p, d_jobs, nj, n, step0, nsteps, s, flux);
   if (variant != 0 && fft1d_r16_enabled(n))

@@ -297,6 +297,7 @@ bool fft3d_supported(Precision p, int n) {
 
 cudaError_t launch_fft3d_pass(Precision p, const Fft3dPass &q, int variant, const double *kx2,
                               const void *tw16, const void *wn, cudaStream_t s) {
+  if (mixed_plan(q.n, nullptr)) return launch_fft3d_mixed(p, q, kx2, s);
   if (q.n & (q.n - 1)) return launch_fft3d_bluestein(p, q, kx2, s);
   if (variant == 3) {
     if (fft3d_lines_supported(p, q.n) && wn != nullptr) return launch_fft3d_lines(p, q, kx2, wn, s);

@@ -71,6 +71,23 @@ __device__ __forceinline__ double2 cx_scale_rn(double2 a, double s) {
 __device__ __forceinline__ double2 cx_div_real_rn(double2 a, double s) {
   return mk(__ddiv_rn(a.x, s), __ddiv_rn(a.y, s));
 }
+// a / s for many a and one s: r = 1/s rounded, then one residual correction of
+// a * r (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34(1), 1990): the division's value
+// in three operations instead of a subroutine.  Infinities and NaN pass
+// through as they do in a division.
+struct Divisor {
+  double s, r;
+};
+__device__ __forceinline__ Divisor divisor(double s) { return {s, __ddiv_rn(1.0, s)}; }
+__device__ __forceinline__ double div_by(double a, Divisor d) {
+  const double q = __dmul_rn(a, d.r);
+  const double c = __fma_rn(__fma_rn(-d.s, q, a), d.r, q);
+  return fabs(q) <= 1.7976931348623157e308 ? c : q;
+}
+__device__ __forceinline__ double2 cx_div_by(double2 a, Divisor d) {
+  return mk(div_by(a.x, d), div_by(a.y, d));
+}
 // Smith's complex division (a / b) with the branch on |b.x| vs |b.y|.
 __device__ __forceinline__ double2 cx_div_rn(double2 a, double2 b) {
   if (fabs(b.x) < fabs(b.y)) {

@@ -96,6 +96,30 @@ inline bool fft1d_pair_size(Precision p, int n) { return p == kFP64 && n == 1638
 // smallest power of two >= 2n - 1); n itself for powers of two.
 int fft1d_bluestein_m(int n);
 
+// Passes of the mixed-radix transform (fft_mixed.cuh) of length n, in order:
+// radix, butterflies (n / radix), the multiplier that divides a butterfly's
+// index by the pass's sub-transform length, and for radices above 9 where
+// their (cos, sin) factors lie in the table (16 bytes: one load a pass).
+struct MixedPlan {
+  static constexpr int kMaxPasses = 8;
+  struct alignas(16) Pass {
+    int radix, nb;
+    unsigned magic;
+    int rot;
+  };
+  Pass pass[kMaxPasses];
+  int n, passes;
+  int table;  // entries of the table
+  bool big;   // a radix above 13
+};
+// Fills *plan (may be null) and returns true for lengths that are not powers
+// of two and have no prime factor above 31.
+bool mixed_plan(int n, MixedPlan *plan);
+// FFTSolver2D steps of such lengths (fft1d_mixed.cu); the job's twiddle is the
+// plan's table.
+cudaError_t launch_fft1d_mixed(Precision p, const Fft1dJob *d_jobs, int nj, int n, int step0,
+                               int nsteps, cudaStream_t s, bool flux);
+
 // ------------------------------------------------------------ CN 1-D ------
 // Crank-Nicolson problem (CrankNicholson with default F=G=H=1, J=0).
 struct CnJob {
@@ -309,6 +333,7 @@ struct Fft3dPass {
   double stepn_x, stepn_y; // step*n per axis (FFTSolver3D::spatialFreqX/Y)
   // refraction (y pass)
   double k, dz, xmin, dx, ymin, dy, z1, z0, norm;
+  double inv_norm;         // 1/norm, rounded
   int nspheres;
   Csg csg;                 // CSG material (instead of spheres) when csg.active
   // sampled material of this step (instead of spheres or CSG) when
@@ -365,6 +390,9 @@ cudaError_t launch_fft3d_r16(Precision p, const Fft3dPass &q, const double *kx2,
 // fft3d_blu.cu); q.chirp, q.bconv, q.m and q.twiddle as described above.
 cudaError_t launch_fft3d_bluestein(Precision p, const Fft3dPass &q, const double *kx2,
                                    cudaStream_t s);
+// Line passes of lengths that mixed_plan takes (fft3d_mixed.cu); q.twiddle is
+// the plan's pass-ordered table.
+cudaError_t launch_fft3d_mixed(Precision p, const Fft3dPass &q, const double *kx2, cudaStream_t s);
 cudaError_t launch_fft3d_lines(Precision p, const Fft3dPass &q, const double *kx2, const void *wn,
                                cudaStream_t s);
 // Bounded waits of the line-pass kernels that ran out on the current device.
