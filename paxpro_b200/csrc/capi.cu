@@ -512,7 +512,8 @@ int fft1d_setup(pxp_solver_s *h) {
   } else if ((rc = shared_table(h, 0, &h->d_tw))) {
     return rc;
   }
-  if (pxp::fft1d_r16_enabled((int)h->nx) && (rc = shared_table(h, 4, &h->d_wn))) return rc;
+  if ((pxp::fft1d_r16_enabled(h->prec, (int)h->nx) || pxp::fft1d_r8_enabled(h->prec, (int)h->nx)) &&
+      (rc = shared_table(h, 4, &h->d_wn))) return rc;
   return alloc(h, &h->d_job, sizeof(pxp::Fft1dJob), "job descriptor");
 }
 
@@ -1105,30 +1106,26 @@ int fft3d_variant(pxp_solver_s *h, const pxp::Fft3dPass &q0, const void *kx2, co
   return PXP_OK;
 }
 
-// Launch-variant tuner of the 2-D step kernels: FFTSolver2D at 512..4096
-// points (shared-memory Stockham kernel or register-resident radix-16
-// kernel) and CrankNicholson's step-invariant path at 4096 rows (one CTA or
-// a cluster of two).  As for FFTSolver3D, the first solver with a given
-// (device, precision, kind, size) times every variant on a scratch copy of
-// its own job (zeroed field; no saves, flux sums or per-step tables; 64
+// Launch-variant tuner of CrankNicholson's step-invariant path at 4096 rows
+// (one CTA or a cluster of two).  As for FFTSolver3D, the first solver with a
+// given (device, precision, kind, size) times every variant on a scratch copy
+// of its own job (zeroed field; no saves, flux sums or per-step tables; 64
 // steps a launch, three rounds of an untimed launch and a timed one, the
-// fastest kept) and every
-// solver with that key -- alone or in a batch -- runs the winner from its
-// first step, so a field never depends on when tuning ran (the variants
-// agree within the FP64 tolerance, not bit for bit).  PXP_FFT1D_R16=0|1 and
-// PXP_CN_CLUSTER=0|1 pin the variant instead.
+// fastest kept) and every solver with that key -- alone or in a batch -- runs
+// the winner from its first step, so a field never depends on when tuning ran
+// (the variants agree within the FP64 tolerance, not bit for bit).
+// PXP_CN_CLUSTER=0|1 pins the variant instead.
 std::map<std::tuple<int, int, int, unsigned>, int> g_2d_variant;
 
 bool cn_uses_const(const pxp_solver_s *h);
 
 int variant_2d(pxp_solver_s *h, int *out) {
   *out = -1;
-  const bool fft = h->prob.kind == PXP_FFT_SOLVER_2D;
-  if (!fft && !(h->prob.kind == PXP_CRANK_NICHOLSON && cn_uses_const(h))) return PXP_OK;
-  const int n = fft ? (int)h->nx : pxp::cn_padded_n((int)h->nx);
-  const int nv = fft ? pxp::fft1d_variants(h->prec, n) : pxp::cn_const_variants(h->prec, n);
+  if (h->prob.kind != PXP_CRANK_NICHOLSON || !cn_uses_const(h)) return PXP_OK;
+  const int n = pxp::cn_padded_n((int)h->nx);
+  const int nv = pxp::cn_const_variants(h->prec, n);
   if (nv < 2) return PXP_OK;
-  if (const char *env = std::getenv(fft ? "PXP_FFT1D_R16" : "PXP_CN_CLUSTER")) {
+  if (const char *env = std::getenv("PXP_CN_CLUSTER")) {
     if (env[0] == '0' || env[0] == '1') {
       *out = env[0] - '0';
       return PXP_OK;
@@ -1141,7 +1138,7 @@ int variant_2d(pxp_solver_s *h, int *out) {
     *out = it->second;
     return PXP_OK;
   }
-  const size_t job_bytes = fft ? sizeof(pxp::Fft1dJob) : sizeof(pxp::CnJob);
+  const size_t job_bytes = sizeof(pxp::CnJob);
   const size_t field_bytes = h->csize * (size_t)n;
   void *scratch = nullptr, *djob = nullptr;
   cudaError_t e = cudaMallocAsync(&scratch, field_bytes, h->stream);
@@ -1150,24 +1147,14 @@ int variant_2d(pxp_solver_s *h, int *out) {
     if (scratch) cudaFreeAsync(scratch, h->stream);
     return h->cuda_fail(e, "2-D kernel tuning scratch");
   }
-  pxp::Fft1dJob jf = h->job_fft;
   pxp::CnJob jc = h->job_cn;
-  if (fft) {
-    jf.field = scratch;
-    jf.saves = nullptr;
-    jf.save_every = 0;
-    jf.trans_stride = 0;
-    jf.flux = pxp::FluxSpec{};
-  } else {
-    jc.field = scratch;
-    jc.saves = nullptr;
-    jc.save_every = 0;
-    jc.flux = pxp::FluxSpec{};
-  }
+  jc.field = scratch;
+  jc.saves = nullptr;
+  jc.save_every = 0;
+  jc.flux = pxp::FluxSpec{};
   e = cudaMemsetAsync(scratch, 0, field_bytes, h->stream);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(djob, fft ? (const void *)&jf : (const void *)&jc, job_bytes,
-                        cudaMemcpyHostToDevice, h->stream);
+    e = cudaMemcpyAsync(djob, &jc, job_bytes, cudaMemcpyHostToDevice, h->stream);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (e == cudaSuccess) e = cudaEventCreate(&e0);
   if (e == cudaSuccess) e = cudaEventCreate(&e1);
@@ -1175,10 +1162,8 @@ int variant_2d(pxp_solver_s *h, int *out) {
   float best = 1e30f;
   constexpr int kTuneSteps = 64;
   auto launch_v = [&](int v) {
-    return fft ? pxp::launch_fft1d(h->prec, (const pxp::Fft1dJob *)djob, 1, n, 1, kTuneSteps,
-                                   h->stream, false, v)
-               : pxp::launch_cn_const(h->prec, (const pxp::CnJob *)djob, 1, n, 1, kTuneSteps,
-                                      h->stream, false, v);
+    return pxp::launch_cn_const(h->prec, (const pxp::CnJob *)djob, 1, n, 1, kTuneSteps, h->stream,
+                                false, v);
   };
   for (int v = 0; v < nv && e == cudaSuccess; ++v) {
     float tmin = 1e30f;
@@ -1864,13 +1849,10 @@ int pxp_step(pxp_solver h, int nsteps) {
                                         " are outside the material planes provided");
   cudaError_t e = cudaSuccess;
   switch (h->prob.kind) {
-    case PXP_FFT_SOLVER_2D: {
-      int v = -1;
-      if (int rc = variant_2d(h, &v)) return rc;
+    case PXP_FFT_SOLVER_2D:
       e = pxp::launch_fft1d(h->prec, (const pxp::Fft1dJob *)h->d_job, 1, (int)h->nx,
-                            (int)first, nsteps, h->stream, h->flux_count > 0, v);
+                            (int)first, nsteps, h->stream, h->flux_count > 0);
       break;
-    }
     case PXP_CRANK_NICHOLSON:
       if (!(h->cn_const && !h->prob.transparent_bc && h->mat_stride == 0) &&
           !pxp::cn_supported(h->prec, (int)h->nx))
@@ -2675,8 +2657,7 @@ int pxp_batch_round(pxp_batch b, int max_steps) {
       e = cudaMemsetAsync(b->d_queue + gi, 0, sizeof(unsigned), gst);
       if (e == cudaSuccess)
         e = pxp::launch_fft1d((pxp::Precision)k.prec, (const pxp::Fft1dJob *)jobs,
-                              (int)list.size(), k.n, -1, -1, gst, any_flux, variant,
-                              b->d_queue + gi);
+                              (int)list.size(), k.n, -1, -1, gst, any_flux, b->d_queue + gi);
     }
     else if (k.cpath)
       e = pxp::launch_cn_const((pxp::Precision)k.prec, (const pxp::CnJob *)jobs, (int)list.size(),

@@ -23,10 +23,16 @@ namespace pxp {
 // Per-step factor tables: complex128 in FP64 mode, which reproduces the
 // reference's rounding (rounded complex product, then division by N);
 // split complex64 pairs of t/N in FP32 served mode (one FMA chain).
-__device__ __forceinline__ void refract(double2 &u, double2 t, double n) {
-  u = cx_div_real_rn(cx_mul_rn(u, t), n);
+// (u * t) / N: for a power of two the product with its exact reciprocal rounds
+// as the division does.
+__device__ __forceinline__ void refract(double2 &u, double2 t, double inv_n) {
+  u = cx_scale_rn(cx_mul_rn(u, t), inv_n);
 }
 __device__ __forceinline__ void refract(float2 &u, float4 t, float) { u = tw_mul(u, t); }
+__device__ __forceinline__ void refract(double2 &u, double2 t, Divisor n) {
+  u = cx_div_by(cx_mul_rn(u, t), n);
+}
+__device__ __forceinline__ void refract(float2 &u, float4 t, Divisor) { u = tw_mul(u, t); }
 __device__ __forceinline__ double2 kmul(double2 u, double2 k) { return cx_mul_rn(u, k); }
 __device__ __forceinline__ float2 kmul(float2 u, float4 k) { return tw_mul(u, k); }
 
@@ -60,7 +66,7 @@ __global__ void __launch_bounds__(T) fft1d_kernel(const Fft1dJob *__restrict__ j
   const W *kern = reinterpret_cast<const W *>(job.kern);
   const W *trans0 = reinterpret_cast<const W *>(job.trans);
   C *saves = reinterpret_cast<C *>(job.saves);
-  const R nreal = (R)N;
+  const R inv_n = (R)1 / (R)N;
   for (int s = 0; s < job.nsteps; ++s) {
     const int step = job.step0 + s;
     // this step's flux window, loaded early so its latency hides behind the step
@@ -77,7 +83,7 @@ __global__ void __launch_bounds__(T) fft1d_kernel(const Fft1dJob *__restrict__ j
     double acc = 0.0;
     for (int i = lane; i < N; i += T) {
       C v = u[sw<C>(i)];
-      refract(v, trans[i], nreal);
+      refract(v, trans[i], inv_n);
       u[sw<C>(i)] = v;
       if (save) slot[i] = v;
       if (flux) flux_add(acc, i, fw, to_d(v));
@@ -115,7 +121,7 @@ __global__ void __launch_bounds__(T) fft1d_bluestein_kernel(const Fft1dJob *__re
   const W *kern = reinterpret_cast<const W *>(job.kern);
   const W *trans0 = reinterpret_cast<const W *>(job.trans);
   C *saves = reinterpret_cast<C *>(job.saves);
-  const R nreal = (R)n;
+  const Divisor nreal = divisor((double)n);
   for (int s = 0; s < job.nsteps; ++s) {
     const int step = job.step0 + s;
     int2 fw;
@@ -224,26 +230,21 @@ static cudaError_t launch_nf(const Fft1dJob *d_jobs, int nj, int step0, int nste
               : launch_n<R, N, false>(d_jobs, nj, step0, nsteps, s, queue);
 }
 
-int fft1d_variants(Precision p, int n) {
-  return !fft1d_pair_size(p, n) && fft1d_r16_enabled(n) ? 2 : 1;
-}
-
 cudaError_t launch_fft1d(Precision p, const Fft1dJob *d_jobs, int nj, int n, int step0,
-                         int nsteps, cudaStream_t s, bool flux, int variant, unsigned *queue) {
+                         int nsteps, cudaStream_t s, bool flux, unsigned *queue) {
   if (nj <= 0) return cudaSuccess;
   if (mixed_plan(n, nullptr))
     return launch_fft1d_mixed(p, d_jobs, nj, n, step0, nsteps, s, flux);
   if (n & (n - 1)) return launch_bluestein(p, d_jobs, nj, n, step0, nsteps, s, flux);
   if (fft1d_pair_size(p, n)) return launch_fft1d_pair(p, d_jobs, nj, n, step0, nsteps, s, flux);
-  if (variant != 0 && fft1d_r16_enabled(n))
-    return launch_fft1d_r16(p, d_jobs, nj, n, step0, nsteps, s, flux, queue);
+  if (fft1d_r8_enabled(p, n)) return launch_fft1d_r8(p, d_jobs, nj, n, step0, nsteps, s, flux, queue);
+  if (fft1d_r16_enabled(p, n)) return launch_fft1d_r16(d_jobs, nj, step0, nsteps, s, flux, queue);
 #define PXP_CASE(NN)                                                              \
   case NN:                                                                        \
     return p == kFP64 ? launch_nf<double, NN>(d_jobs, nj, step0, nsteps, s, flux, queue)     \
                       : launch_nf<float, NN>(d_jobs, nj, step0, nsteps, s, flux, queue);
   switch (n) {
-    PXP_CASE(8) PXP_CASE(16) PXP_CASE(32) PXP_CASE(64) PXP_CASE(128) PXP_CASE(256)
-    PXP_CASE(512) PXP_CASE(1024) PXP_CASE(2048) PXP_CASE(4096) PXP_CASE(8192)
+    PXP_CASE(8) PXP_CASE(16) PXP_CASE(32) PXP_CASE(8192)
     case 16384:
       if (p == kFP32) return launch_nf<float, 16384>(d_jobs, nj, step0, nsteps, s, flux, queue);
       return cudaErrorInvalidValue;

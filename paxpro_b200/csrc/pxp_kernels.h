@@ -59,32 +59,32 @@ struct Fft1dJob {
   const void *chirp;
   const void *bconv;
   int m;
-  // powers of two 512 .. 4096 (fft1d_r16.cu): N entries exp(-2 pi i m / N)
+  // powers of two 64 .. 4096 (fft1d_r16.cu, fft1d_r8.cu): N entries exp(-2 pi i m / N)
   const void *wn;
 };
 
 // Launch nj jobs that all share one transform length n (one CTA per job).
 // step0/nsteps >= 0 override every job's own values (single-problem use).
 // flux: some job has flux windows (the kernel variant that sums them).
-// Register-resident radix-16 FFTSolver2D kernel (fft1d_r16.cu): whether it
-// takes size n (powers of two 512 .. 4096), and its launch.
-bool fft1d_r16_enabled(int n);
-cudaError_t launch_fft1d_r16(Precision p, const Fft1dJob *d_jobs, int nj, int n, int step0,
-                             int nsteps, cudaStream_t s, bool flux, unsigned *queue = nullptr);
-// Launch variants of the 2-D step kernels, chosen per (device, precision,
-// size) by the tuner in capi.cu: FFTSolver2D 0 = shared-memory Stockham
-// kernel, 1 = register-resident radix-16 kernel; CrankNicholson's
-// step-invariant path at 4096 rows 0 = one CTA, 1 = a cluster of two CTAs.
-// *_variants returns how many a size has (1: nothing to choose); variant
-// -1 is the default (the radix-16 kernel where it runs; one CTA).
-int fft1d_variants(Precision p, int n);
+// Register-resident FFTSolver2D kernels: 8 points a thread (fft1d_r8.cu; powers
+// of two 64 .. 2048, in FP32 to 4096) and 16 (fft1d_r16.cu; FP64 4096).
+bool fft1d_r8_enabled(Precision p, int n);
+cudaError_t launch_fft1d_r8(Precision p, const Fft1dJob *d_jobs, int nj, int n, int step0,
+                            int nsteps, cudaStream_t s, bool flux, unsigned *queue = nullptr);
+bool fft1d_r16_enabled(Precision p, int n);
+cudaError_t launch_fft1d_r16(const Fft1dJob *d_jobs, int nj, int step0, int nsteps, cudaStream_t s,
+                             bool flux, unsigned *queue = nullptr);
+// Launch variants of CrankNicholson's step-invariant path, chosen per (device,
+// precision, size) by the tuner in capi.cu: at 4096 rows 0 = one CTA, 1 = a
+// cluster of two CTAs.  Returns how many a size has (1: nothing to choose);
+// variant -1 is the default (one CTA).
 int cn_const_variants(Precision p, int n);
 // queue: a device counter (zero at launch) that makes the power-of-two
 // kernels persistent -- at most one wave of CTAs, each taking its next job
 // from the counter (persistent.cuh); null: one CTA per job.
 cudaError_t launch_fft1d(Precision p, const Fft1dJob *d_jobs, int nj, int n,
                          int step0, int nsteps, cudaStream_t s, bool flux = false,
-                         int variant = -1, unsigned *queue = nullptr);
+                         unsigned *queue = nullptr);
 bool fft1d_supported(Precision p, int n);
 // complex128 lines of 16384 points (fft1d_pair.cu): a cluster of two CTAs per
 // job, each holding the points of one parity; the job's twiddle is the
