@@ -78,6 +78,9 @@ struct pxp_solver_s {
   void *d_lu = nullptr;                      // factor tables of step-invariant matrices
   int adi_tab_run[2][2] = {};                // x / y staged ADI tables: identical chunks
   bool cn_const = false;                     // CN matrix step-invariant
+  bool cn_two_planes = false;                // its one step's two planes differ
+  bool cn_vacuum = false;                    // no material set yet: its tables are built
+                                             // when it steps without one
   size_t dev_bytes = 0;                      // device memory held by the handle
   pxp::Fft1dJob job_fft{};                   // host copies of the job descriptors
   pxp::CnJob job_cn{};
@@ -592,9 +595,10 @@ int cn_set_planes(pxp_solver_s *h, const double *delta, const double *beta, int 
   h->material_set = true;
   // step-invariant matrix when the same plane serves every step
   h->cn_const = false;
+  h->cn_two_planes = std::memcmp(&buf[0], &buf[2 * per], sizeof(double) * 2 * per) != 0;
   if (nsteps == 1 && pxp::cn_const_supported(h->prec, pxp::cn_padded_n((int)n))) {
-    int rc2 = cn_build_lu(h, delta, beta);
-    if (rc2) return rc2;
+    if (!h->cn_vacuum)
+      if (int rc2 = cn_build_lu(h, delta, beta)) return rc2;
     h->cn_const = true;
   }
   return PXP_OK;
@@ -631,13 +635,38 @@ int cn_build_lu(pxp_solver_s *h, const double *delta, const double *beta) {
   for (unsigned i = 0; i < n; ++i)
     diag[i] = fval * 1.0 + 0.25 * (Hp + Hm) * gval * IMAG_UNIT * rho +
               0.5 * (beta[i] * r + IMAG_UNIT * delta[i] * r);
-  const cd sub = -0.25 * IMAG_UNIT * rho * Hm * gval;
-  std::vector<cd> gh;
-  thomas_factor(diag, sub, gh);
+  // pivots from both ends (cn.cu) in extended precision: a rounding error of a
+  // table entry is the same at every step
+  struct Lc {
+    long double re, im;
+  };
+  const long double q = 0.25L * (long double)rho;  // off-diagonal -i q
+  auto recip = [](Lc z) {
+    const long double m = 1.0L / (z.re * z.re + z.im * z.im);
+    return Lc{z.re * m, -z.im * m};
+  };
+  // b - (-i q)^2 / pivot = b + q^2 / pivot
+  auto next = [q](cd b, Lc inv) { return Lc{b.real() + q * q * inv.re, b.imag() + q * q * inv.im}; };
+  std::vector<cd> tabs(3 * (size_t)np);  // hL, hR, 2 w
+  std::vector<Lc> left(np);
+  Lc inv{0.0L, 0.0L};
+  for (unsigned i = 0; i < np; ++i) {
+    tabs[i] = cd((double)(-q * inv.im), (double)(q * inv.re));  // i q / previous pivot
+    left[i] = next(diag[i], inv);
+    inv = recip(left[i]);
+  }
+  inv = Lc{0.0L, 0.0L};
+  for (unsigned i = np; i-- > 0;) {
+    tabs[np + i] = cd((double)(-q * inv.im), (double)(q * inv.re));
+    const Lc right = next(diag[i], inv);
+    inv = recip(right);
+    const Lc w = recip(Lc{left[i].re + right.re - diag[i].real(), left[i].im + right.im - diag[i].imag()});
+    tabs[2 * (size_t)np + i] = cd((double)(2.0L * w.re), (double)(2.0L * w.im));
+  }
   free_dev(h->d_lu, h->stream);
   int rc;
-  if ((rc = alloc(h, &h->d_lu, sizeof(cd) * 2 * np, "factor tables"))) return rc;
-  if (int rc_ = h2d(h, h->d_lu, gh.data(), sizeof(cd) * 2 * np)) return rc_;
+  if ((rc = alloc(h, &h->d_lu, sizeof(cd) * tabs.size(), "factor tables"))) return rc;
+  if (int rc_ = h2d(h, h->d_lu, tabs.data(), sizeof(cd) * tabs.size())) return rc_;
   return PXP_OK;
 }
 
@@ -1106,92 +1135,18 @@ int fft3d_variant(pxp_solver_s *h, const pxp::Fft3dPass &q0, const void *kx2, co
   return PXP_OK;
 }
 
-// Launch-variant tuner of CrankNicholson's step-invariant path at 4096 rows
-// (one CTA or a cluster of two).  As for FFTSolver3D, the first solver with a
-// given (device, precision, kind, size) times every variant on a scratch copy
-// of its own job (zeroed field; no saves, flux sums or per-step tables; 64
-// steps a launch, three rounds of an untimed launch and a timed one, the
-// fastest kept) and every solver with that key -- alone or in a batch -- runs
-// the winner from its first step, so a field never depends on when tuning ran
-// (the variants agree within the FP64 tolerance, not bit for bit).
-// PXP_CN_CLUSTER=0|1 pins the variant instead.
-std::map<std::tuple<int, int, int, unsigned>, int> g_2d_variant;
-
 bool cn_uses_const(const pxp_solver_s *h);
 
-int variant_2d(pxp_solver_s *h, int *out) {
-  *out = -1;
-  if (h->prob.kind != PXP_CRANK_NICHOLSON || !cn_uses_const(h)) return PXP_OK;
-  const int n = pxp::cn_padded_n((int)h->nx);
-  const int nv = pxp::cn_const_variants(h->prec, n);
-  if (nv < 2) return PXP_OK;
-  if (const char *env = std::getenv("PXP_CN_CLUSTER")) {
-    if (env[0] == '0' || env[0] == '1') {
-      *out = env[0] - '0';
-      return PXP_OK;
-    }
-  }
-  const auto key = std::make_tuple(h->prob.device, (int)h->prec, (int)h->prob.kind, (unsigned)n);
-  std::lock_guard<std::mutex> lk(g_tune_mutex);
-  auto it = g_2d_variant.find(key);
-  if (it != g_2d_variant.end()) {
-    *out = it->second;
-    return PXP_OK;
-  }
-  const size_t job_bytes = sizeof(pxp::CnJob);
-  const size_t field_bytes = h->csize * (size_t)n;
-  void *scratch = nullptr, *djob = nullptr;
-  cudaError_t e = cudaMallocAsync(&scratch, field_bytes, h->stream);
-  if (e == cudaSuccess) e = cudaMallocAsync(&djob, job_bytes, h->stream);
-  if (e != cudaSuccess) {
-    if (scratch) cudaFreeAsync(scratch, h->stream);
-    return h->cuda_fail(e, "2-D kernel tuning scratch");
-  }
-  pxp::CnJob jc = h->job_cn;
-  jc.field = scratch;
-  jc.saves = nullptr;
-  jc.save_every = 0;
-  jc.flux = pxp::FluxSpec{};
-  e = cudaMemsetAsync(scratch, 0, field_bytes, h->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(djob, &jc, job_bytes, cudaMemcpyHostToDevice, h->stream);
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
-  if (e == cudaSuccess) e = cudaEventCreate(&e0);
-  if (e == cudaSuccess) e = cudaEventCreate(&e1);
-  int best_v = 0;
-  float best = 1e30f;
-  constexpr int kTuneSteps = 64;
-  auto launch_v = [&](int v) {
-    return pxp::launch_cn_const(h->prec, (const pxp::CnJob *)djob, 1, n, 1, kTuneSteps, h->stream,
-                                false, v);
-  };
-  for (int v = 0; v < nv && e == cudaSuccess; ++v) {
-    float tmin = 1e30f;
-    for (int rep = 0; rep < 3 && e == cudaSuccess; ++rep) {
-      e = launch_v(v);  // untimed: the device is busy while the timed launch is prepared
-      cudaEventRecord(e0, h->stream);
-      if (e == cudaSuccess) e = launch_v(v);
-      cudaEventRecord(e1, h->stream);
-      if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-      float ms = 0.f;
-      if (e == cudaSuccess && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess)
-        tmin = std::min(tmin, ms);
-    }
-    if (tmin < best) {
-      best = tmin;
-      best_v = v;
-    }
-  }
-  // the job descriptor must stay valid until the launches that read it ran
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  if (e0) cudaEventDestroy(e0);
-  if (e1) cudaEventDestroy(e1);
-  cudaFreeAsync(djob, h->stream);
-  cudaFreeAsync(scratch, h->stream);
-  if (e != cudaSuccess) return h->cuda_fail(e, "2-D kernel tuning");
-  g_2d_variant[key] = best_v;
-  *out = best_v;
-  return PXP_OK;
+int cn_write_job(pxp_solver_s *h);
+
+// A CrankNicholson solver that steps before any material is set: its vacuum
+// tables.
+int cn_vacuum_tables(pxp_solver_s *h) {
+  if (!h->cn_vacuum || !cn_uses_const(h)) return PXP_OK;
+  const std::vector<double> zeros(h->npts, 0.0);
+  if (int rc = cn_build_lu(h, zeros.data(), zeros.data())) return rc;
+  h->cn_vacuum = false;
+  return cn_write_job(h);
 }
 
 int fft3d_steps(pxp_solver_s *h, unsigned first, int nsteps) {
@@ -1334,8 +1289,13 @@ int cn_write_job(pxp_solver_s *h) {
   j.max_slots = h->max_slots;
   j.mat_step0 = h->mat_step0;
   j.transparent = h->prob.transparent_bc ? 1 : 0;
-  j.lu_g = h->d_lu;
-  j.lu_h = h->d_lu ? (const void *)((const cd *)h->d_lu + pxp::cn_padded_n((int)n)) : nullptr;
+  j.two_planes = h->cn_two_planes ? 1 : 0;
+  if (h->d_lu) {
+    const cd *lu = (const cd *)h->d_lu;
+    j.lu_l = lu;
+    j.lu_r = lu + pxp::cn_padded_n((int)n);
+    j.lu_w = lu + 2 * pxp::cn_padded_n((int)n);
+  }
   j.flux = pxp::FluxSpec{h->d_flux_win, h->d_flux, h->flux_step0, h->flux_count};
   h->job_cn = j;
   if (int rc_ = h2d(h, h->d_job, &j, sizeof(j))) return rc_;
@@ -1485,6 +1445,7 @@ int pxp_solver_create(const pxp_problem *problem, pxp_solver *out) {
       break;
     case PXP_CRANK_NICHOLSON:
       if ((rc = alloc(h, &h->d_job, sizeof(pxp::CnJob), "job descriptor"))) return cleanup_fail(rc);
+      h->cn_vacuum = true;
       if ((rc = cn_set_planes(h, zeros.data(), zeros.data(), 1, 1, false))) return cleanup_fail(rc);
       if ((rc = cn_write_job(h))) return cleanup_fail(rc);
       break;
@@ -1590,6 +1551,7 @@ int pxp_set_material_table(pxp_solver h, const double *delta, const double *beta
       if ((rc = fft1d_set_trans(h, delta, beta, 1, 1))) return rc;
       break;
     case PXP_CRANK_NICHOLSON:
+      h->cn_vacuum = false;
       if ((rc = cn_set_planes(h, delta, beta, 1, 1, false))) return rc;
       break;
     case PXP_FFT_SOLVER_3D:
@@ -1622,6 +1584,7 @@ int pxp_set_material_planes(pxp_solver h, const double *delta, const double *bet
       if (nsteps == 1) h->trans_stride = 0;
       break;
     case PXP_CRANK_NICHOLSON:
+      h->cn_vacuum = false;
       if ((rc = cn_set_planes(h, delta, beta, nsteps, first_step, true))) return rc;
       break;
     case PXP_FFT_SOLVER_3D:
@@ -1854,18 +1817,16 @@ int pxp_step(pxp_solver h, int nsteps) {
                             (int)first, nsteps, h->stream, h->flux_count > 0);
       break;
     case PXP_CRANK_NICHOLSON:
-      if (!(h->cn_const && !h->prob.transparent_bc && h->mat_stride == 0) &&
+      if (int rc = cn_vacuum_tables(h)) return rc;
+      if (!cn_uses_const(h) &&
           !pxp::cn_supported(h->prec, (int)h->nx))
         return h->fail(PXP_ERR_UNSUPPORTED,
                        "CrankNicholson at " + std::to_string(h->nx) +
                            " points runs with a z-invariant medium and Dirichlet ends only");
-      if (h->cn_const && !h->prob.transparent_bc && h->mat_stride == 0) {
-        int v = -1;
-        if (int rc = variant_2d(h, &v)) return rc;
+      if (cn_uses_const(h))
         e = pxp::launch_cn_const(h->prec, (const pxp::CnJob *)h->d_job, 1,
                                  pxp::cn_padded_n((int)h->nx), (int)first, nsteps, h->stream,
-                                 h->flux_count > 0, v);
-      }
+                                 h->flux_count > 0);
       else
         e = pxp::launch_cn(h->prec, (const pxp::CnJob *)h->d_job, 1, pxp::cn_padded_n((int)h->nx),
                            (int)first, nsteps, h->stream, h->flux_count > 0);
@@ -2528,6 +2489,8 @@ int pxp_batch_admit(pxp_batch b, pxp_solver h, int nsteps) {
       (h->current_step < (unsigned)h->plane_first ||
        (long long)h->current_step + nsteps > (long long)h->plane_first + h->plane_count))
     return b->fail(PXP_ERR_INVALID, "steps outside the material planes provided");
+  if (h->prob.kind == PXP_CRANK_NICHOLSON)
+    if (int rc = cn_vacuum_tables(h)) return b->fail(rc, h->err);
   if (h->prob.kind == PXP_CRANK_NICHOLSON && !cn_uses_const(h) &&
       !pxp::cn_supported(h->prec, (int)h->nx))
     return b->fail(PXP_ERR_UNSUPPORTED, "CrankNicholson at this size needs a z-invariant medium "
@@ -2571,15 +2534,6 @@ int pxp_batch_round(pxp_batch b, int max_steps) {
                        return std::min(a->batch_remaining, max_steps) >
                               std::min(c->batch_remaining, max_steps);
                      });
-  // each group's kernel variant, the one every solver of its key runs alone
-  // (tuned here, before this round launches anything, if no solver of the
-  // key has stepped yet)
-  std::vector<int> gvariant;
-  for (auto &g : groups) {
-    int v = -1;
-    if (int rc = variant_2d(g.second.front(), &v)) return b->fail(rc, g.second.front()->err);
-    gvariant.push_back(v);
-  }
   size_t total = 0;
   for (auto &g : groups)
     total += g.second.size() * (g.first.kind == PXP_FFT_SOLVER_2D ? sizeof(pxp::Fft1dJob) : sizeof(pxp::CnJob));
@@ -2651,7 +2605,6 @@ int pxp_batch_round(pxp_batch b, int max_steps) {
     const void *jobs = (const char *)b->d_jobs + o.first;
     bool any_flux = false;
     for (const pxp_solver_s *h : list) any_flux = any_flux || h->flux_count > 0;
-    const int variant = gvariant[gi];
     cudaError_t e;
     if (k.kind == PXP_FFT_SOLVER_2D) {
       e = cudaMemsetAsync(b->d_queue + gi, 0, sizeof(unsigned), gst);
@@ -2661,7 +2614,7 @@ int pxp_batch_round(pxp_batch b, int max_steps) {
     }
     else if (k.cpath)
       e = pxp::launch_cn_const((pxp::Precision)k.prec, (const pxp::CnJob *)jobs, (int)list.size(),
-                               pxp::cn_padded_n(k.n), -1, -1, gst, any_flux, variant);
+                               pxp::cn_padded_n(k.n), -1, -1, gst, any_flux);
     else
       e = pxp::launch_cn((pxp::Precision)k.prec, (const pxp::CnJob *)jobs, (int)list.size(),
                          pxp::cn_padded_n(k.n), -1, -1, gst, any_flux);

@@ -25,7 +25,6 @@
 #include "pxp_kernels.h"
 #include <cooperative_groups.h>
 
-#include "scan_solve.cuh"
 #include "tridiag.cuh"
 
 namespace cg = cooperative_groups;
@@ -181,181 +180,238 @@ __global__ void __launch_bounds__(T) cn_kernel(const CnJob *__restrict__ jobs, i
   for (int i = t; i < nreal; i += T) field[i] = u[i];
 }
 
-// z-invariant medium, Dirichlet ends: the step matrix is fixed, so the
-// factor tables g, h (host-computed) are loaded into shared memory once and
-// each step is the right-hand-side stencil plus two substitution scans
-// (scan_solve.cuh).  The field stays in registers: thread t owns points
-// t*M .. t*M+M-1 and trades its two edge values with its neighbours through
-// shared memory.  The right-hand side is regrouped as
-// i*q*(left + right) + d*centre, q = rho/4, with the per-point coefficient
-// d = (1 - 0.5*(beta'*r + i*delta'*r)) - i*rho/2 formed once (the first part
-// with the reference's rounding) and kept in shared memory; the regrouping
-// and the FMAs differ from the reference's operation order at rounding level.
-// Tables sit in chunk-transposed slots (cslot), free of bank conflicts.
-template <typename R, int M, int T, bool FLUX>
+// Dirichlet ends: the step as one solve.  With A the step's matrix (diagonal
+// 1 + i rho/2 + m, off-diagonal s = -i rho/4, m = (beta r + i delta r)/2 at the
+// new plane) and m' the old plane's, the right-hand side's matrix is 2 - A +
+// (m - m'), so
+//   u_new = A^-1 ((2 + m - m') u) - u:
+// no stencil, no halo exchange, a pointwise right-hand side (a constant 2 when
+// the medium does not change along z).
+//
+// A is solved from both ends at once (D. J. Evans and M. Hatzopoulos, "A
+// parallel linear system solver", Int. J. Comput. Math. 7(3), 1979): with the
+// pivots d_i = b_i - s^2/d_(i-1) from the left and e_i = b_i - s^2/e_(i+1) from
+// the right,
+//   l_i = r_i + hL_i l_(i-1),  hL_i = -s/d_(i-1),
+//   p_i = r_i + hR_i p_(i+1),  hR_i = -s/e_(i+1),
+//   x_i = w_i (l_i + p_i - r_i),  w_i = 1/(d_i + e_i - b_i).
+// The two recurrences are independent: their chains, and the scans that carry
+// them across threads, run side by side, where forward and back substitution
+// run one after the other.
+//
+// Thread t of a CTA owns rows t*M .. t*M+M-1 (CTA k of a cluster: k*M*T on).
+// A chunk's transfer is y_out = a y_in + b; a depends on the tables only, so
+// the scan's levels (Kogge-Stone within a warp, then the warps' totals through
+// shared memory, of every CTA of the cluster through distributed shared
+// memory) move only b, with the products of a kept per thread:
+//   lev  the products a lane's scan levels apply (zero where there is no
+//        partner),
+//   ex   the product over the warp's chunks before this one in scan order,
+//   cf   lane v: the product over the warps between warp v and this one
+//        (zero for warps not before it in scan order).
+// The totals' buffer alternates between steps, so a step has one barrier.
+struct ScanCoef {
+  double2 levL[5], levR[5], exL, exR, cfL, cfR;
+};
+
+__device__ __forceinline__ double2 shfl_up_d2(double2 v, int d) {
+  return mk(__shfl_up_sync(0xffffffffu, v.x, d), __shfl_up_sync(0xffffffffu, v.y, d));
+}
+__device__ __forceinline__ double2 shfl_down_d2(double2 v, int d) {
+  return mk(__shfl_down_sync(0xffffffffu, v.x, d), __shfl_down_sync(0xffffffffu, v.y, d));
+}
+__device__ __forceinline__ double2 shfl_xor_d2(double2 v, int d) {
+  return mk(__shfl_xor_sync(0xffffffffu, v.x, d), __shfl_xor_sync(0xffffffffu, v.y, d));
+}
+
+// The products from each thread's chunk products aL, aR; tot: TW warp totals
+// of each direction (shared memory of the calling CTA, gw: this warp's index
+// among all TW).  Every thread of the TW warps calls it; publish(w, L, R)
+// stores a warp's totals where every warp reads them, sync() follows.
+template <int TW, typename Publish, typename Sync>
+__device__ __forceinline__ ScanCoef scan_coef(double2 aL, double2 aR, const double2 *tot, int gw,
+                                              Publish publish, Sync sync) {
+  const int lane = threadIdx.x & 31;
+  const double2 zero = mk(0.0, 0.0), one = mk(1.0, 0.0);
+  ScanCoef c;
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const int d = 1 << k;
+    const double2 oL = shfl_up_d2(aL, d), oR = shfl_down_d2(aR, d);
+    c.levL[k] = lane >= d ? aL : zero;
+    c.levR[k] = lane + d < 32 ? aR : zero;
+    if (lane >= d) aL = cmul(aL, oL);
+    if (lane + d < 32) aR = cmul(aR, oR);
+  }
+  c.exL = shfl_up_d2(aL, 1);
+  if (lane == 0) c.exL = one;
+  c.exR = shfl_down_d2(aR, 1);
+  if (lane == 31) c.exR = one;
+  c.cfL = c.cfR = zero;
+  if constexpr (TW > 1) {
+    if (lane == 31) publish(gw, 0, aL);
+    if (lane == 0) publish(gw, 1, aR);
+    sync();
+    const int v = lane & (TW - 1);
+    if (v < gw) {
+      c.cfL = one;
+      for (int w = v + 1; w < gw; ++w) c.cfL = cmul(c.cfL, tot[w]);
+    }
+    if (v > gw) {
+      c.cfR = one;
+      for (int w = v - 1; w > gw; --w) c.cfR = cmul(c.cfR, tot[TW + w]);
+    }
+  }
+  return c;
+}
+
+// Carry-ins of both recurrences from the chunks' ends bL, bR (zero carry-in).
+template <int TW, typename Publish, typename Sync>
+__device__ __forceinline__ void scan_carry(double2 bL, double2 bR, const ScanCoef &c,
+                                           const double2 *tot, int gw, Publish publish, Sync sync,
+                                           double2 &cL, double2 &cR) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const int d = 1 << k;
+    const double2 oL = shfl_up_d2(bL, d), oR = shfl_down_d2(bR, d);
+    bL = cfma(c.levL[k], oL, bL);
+    bR = cfma(c.levR[k], oR, bR);
+  }
+  cL = shfl_up_d2(bL, 1);
+  cR = shfl_down_d2(bR, 1);
+  if (lane == 0) cL = mk(0.0, 0.0);
+  if (lane == 31) cR = mk(0.0, 0.0);
+  if constexpr (TW > 1) {
+    if (lane == 31) publish(gw, 0, bL);
+    if (lane == 0) publish(gw, 1, bR);
+    sync();
+    const int v = lane & (TW - 1);
+    double2 sL = cmul(c.cfL, tot[v]), sR = cmul(c.cfR, tot[TW + v]);
+#pragma unroll
+    for (int d = 1; d < TW; d <<= 1) {
+      sL = cadd(sL, shfl_xor_d2(sL, d));
+      sR = cadd(sR, shfl_xor_d2(sR, d));
+    }
+    cL = cfma(c.exL, sL, cL);
+    cR = cfma(c.exR, sR, cR);
+  }
+}
+
+// The solve for the M right-hand sides in r: x replaces r.  hL(m), hR(m),
+// w(m): the tables at this thread's row m.
+template <int M, int TW, typename TL, typename TR, typename TWt, typename Publish, typename Sync>
+__device__ __forceinline__ void two_sided_solve(double2 (&r)[M], TL hL, TR hR, TWt w,
+                                                const ScanCoef &c, const double2 *tot, int gw,
+                                                Publish publish, Sync sync) {
+  double2 acc[M];  // l + p - r
+  double2 l = r[0], p = r[M - 1];
+#pragma unroll
+  for (int k = 0; k < M; ++k) {
+    // row k from the left, row M-1-k from the right; an accumulator is set by
+    // the first of the two that reaches it
+    const int i = k, j = M - 1 - k;
+    if (k > 0) l = cfma(hL(i), l, r[i]);
+    double2 q = mk(0.0, 0.0);
+    if (k > 0) {
+      q = cmul(hR(j), p);
+      p = cadd(q, r[j]);
+    }
+    if (i < j) {
+      acc[i] = l;
+      acc[j] = q;
+    } else if (i == j) {
+      acc[i] = cadd(l, q);
+    } else {
+      acc[i] = cadd(acc[i], l);
+      acc[j] = cadd(acc[j], q);
+    }
+  }
+  double2 cL, cR;
+  scan_carry<TW>(l, p, c, tot, gw, publish, sync, cL, cR);
+#pragma unroll
+  for (int k = 0; k < M; ++k) {
+    const int i = k, j = M - 1 - k;
+    cL = cmul(hL(i), cL);
+    cR = cmul(hR(j), cR);
+    acc[i] = cadd(acc[i], cL);
+    acc[j] = cadd(acc[j], cR);
+  }
+#pragma unroll
+  for (int m = 0; m < M; ++m) r[m] = cmul(w(m), acc[m]);
+}
+
+// The rest of a step: u = x - u, rounded to the field's precision, the save
+// and the flux terms of rows s0 ..
+template <typename R, int M>
+__device__ __forceinline__ double cn_finish(const CnJob &job, int step, double2 (&u)[M],
+                                            const double2 (&x)[M], int s0, int nreal, bool flux,
+                                            int2 fw) {
+  using C = typename Cx<R>::T;
+  C *saves = reinterpret_cast<C *>(job.saves);
+  const bool save = job.save_every > 0 && saves != nullptr && (step % job.save_every) == 0 &&
+                    (step / job.save_every - 1) < job.max_slots;
+  C *slot = save ? saves + (long long)(step / job.save_every - 1) * nreal : nullptr;
+  double acc = 0.0;
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    const C v = from_d<R>(csub(x[m], u[m]));
+    u[m] = to_d(v);
+    if (save && s0 + m < nreal) slot[s0 + m] = v;
+    if (flux) flux_add(acc, s0 + m, fw, u[m]);
+  }
+  return acc;
+}
+
+// The flux sum of a step over the K CTAs of a cluster (part: K slots in CTA
+// 0's shared memory).
+template <int T, int K>
+__device__ __forceinline__ void cn_flux(const CnJob &job, int step, double acc, double (*red)[flux_slots<T>()],
+                                        double *part, int rank) {
+  double *row = red[step & 1];
+  flux_warp_total<T>(acc, row);
+  __syncthreads();
+  if constexpr (K == 1) {
+    flux_store<T>(job.flux, step, row);
+  } else {
+    cg::cluster_group cluster = cg::this_cluster();
+    if (threadIdx.x < 32) {
+      double v = threadIdx.x < flux_slots<T>() ? row[threadIdx.x] : 0.0;
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
+      if (threadIdx.x == 0) *cluster.map_shared_rank(part + rank, 0) = v;
+    }
+    cluster.sync();  // every CTA's total is in CTA 0's slots
+    if (rank == 0 && threadIdx.x == 0) {
+      double v = 0.0;
+      for (int j = 0; j < K; ++j) v += part[j];
+      job.flux.out[step - job.flux.step0] = v;
+    }
+    cluster.sync();  // and read, before the next step's
+  }
+}
+
+// z-invariant medium: tables and scan products set up once, the field in
+// registers for all steps.  K CTAs a problem (a cluster when K > 1).
+//
+// What bounds it: the latency of two chunk chains and the scan, then its SMs'
+// FP64 issue (about 30 operations a row and step).  Measured, us a step, before
+// (stencil, then forward and back substitution with (a, b) scans) and now: 256
+// rows 1.4 -> 0.53, 1000 2.0 -> 1.0, 2048 2.7 -> 1.40, 4096 4.6 -> 1.42, 16384
+// 5.8 -> 2.07; FP32 4096 4.3 -> 1.4, 8192 5.7 -> 2.09.  Against an 80-bit
+// Thomas sweep the error after 3000 to 8000 steps fell from 0.1 .. 19e-12 to
+// 0.07 .. 6e-12 (12 guides at 1000, 2048 and 4096 rows).
+template <typename R, int M, int T, int K, bool FLUX>
 __global__ void __launch_bounds__(T) cn_const_kernel(const CnJob *__restrict__ jobs, int step0_ov,
                                                     int nsteps_ov) {
   using C = typename Cx<R>::T;
-  constexpr int N = M * T;
+  constexpr int NC = M * T, W = T / 32, TW = W * K;
+  static_assert(T % 32 == 0 && TW <= 32, "whole warps, one lane a warp total");
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2 *gs = reinterpret_cast<double2 *>(smem_raw);
-  double2 *hs = gs + N;
-  double2 *ds = hs + N;
-  double2 *xch = ds + N;  // 2 per thread
-  Affine *scratch = reinterpret_cast<Affine *>(xch + 2 * T);
-  __shared__ double flux_red[2][flux_slots<T>()];
-  CnJob job = jobs[blockIdx.x];
-  if (nsteps_ov >= 0) {
-    job.step0 = step0_ov;
-    job.nsteps = nsteps_ov;
-  }
-  const int t = threadIdx.x;
-  const double rho = job.rho, r = job.r;
-  const double2 *gt = reinterpret_cast<const double2 *>(job.lu_g);
-  const double2 *ht = reinterpret_cast<const double2 *>(job.lu_h);
-  const double q = __dmul_rn(0.25, rho);
-  const int s0 = t * M;
-  // rows nreal..N-1 pad the system (their factor-table rows were built with
-  // diagonal kCnPad on the host; their right-hand side is zero)
-  const int nreal = job.n_real > 0 ? job.n_real : N;
-  // each thread fills the slots of its own chunk
-#pragma unroll
-  for (int m = 0; m < M; ++m) {
-    const int k = cslot<M, T>(t, m);
-    gs[k] = gt[s0 + m];
-    hs[k] = ht[s0 + m];
-    if (s0 + m < nreal) {
-      const double bp = job.beta_prev[s0 + m], dp = job.delta_prev[s0 + m];
-      const double2 hh = mk(__dmul_rn(0.5, __dmul_rn(bp, r)), __dmul_rn(0.5, __dmul_rn(dp, r)));
-      ds[k] = mk(__dadd_rn(-hh.x, 1.0), __dsub_rn(-hh.y, 0.5 * rho));
-    } else {
-      ds[k] = mk(0.0, 0.0);
-    }
-  }
-  C *field = reinterpret_cast<C *>(job.field);
-  double2 u[M];
-#pragma unroll
-  for (int m = 0; m < M; ++m) u[m] = s0 + m < nreal ? to_d(field[s0 + m]) : mk(0.0, 0.0);
-  C *saves = reinterpret_cast<C *>(job.saves);
-  for (int st = 0; st < job.nsteps; ++st) {
-    const int step = job.step0 + st;
-    // this step's flux window, loaded early so its latency hides behind the step
-    int2 fw;
-    const bool flux = FLUX && flux_window(job.flux, step, fw);
-    xch[2 * t] = u[0];
-    xch[2 * t + 1] = u[M - 1];
-    __syncthreads();
-    const double2 lft = t > 0 ? xch[2 * t - 1] : mk(0.0, 0.0);
-    const double2 rgt = t < T - 1 ? xch[2 * t + 2] : mk(0.0, 0.0);
-    double2 rh[M];
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const double2 left = m > 0 ? u[m - 1] : lft;
-      // the Dirichlet zero beyond the last real row
-      const double2 right = s0 + m + 1 >= nreal ? mk(0.0, 0.0) : (m < M - 1 ? u[m + 1] : rgt);
-      const double2 sum = cadd(left, right);
-      rh[m] = s0 + m < nreal ? cfma(ds[cslot<M, T>(t, m)], u[m], mk(-q * sum.y, q * sum.x))
-                             : mk(0.0, 0.0);
-    }
-    const_solve_reg<M, T>(rh, gs, hs, t, scratch);
-    const bool save = job.save_every > 0 && saves != nullptr && (step % job.save_every) == 0 &&
-                      (step / job.save_every - 1) < job.max_slots;
-    C *slot = save ? saves + (long long)(step / job.save_every - 1) * nreal : nullptr;
-    double acc = 0.0;
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const C v = from_d<R>(rh[m]);
-      u[m] = to_d(v);
-      if (save && s0 + m < nreal) slot[s0 + m] = v;
-      if (flux) flux_add(acc, s0 + m, fw, u[m]);
-    }
-    if (flux) flux_warp_total<T>(acc, flux_red[st & 1]);
-    __syncthreads();  // xch is rewritten next step
-    if (flux) flux_store<T>(job.flux, step, flux_red[st & 1]);
-  }
-#pragma unroll
-  for (int m = 0; m < M; ++m)
-    if (s0 + m < nreal) field[s0 + m] = from_d<R>(u[m]);
-}
-
-// The same step for systems of K * M * T rows (8192 and 16384) on a cluster
-// of K CTAs, one per SM, CTA k holding rows [k*M*T, (k+1)*M*T) with its
-// slice of the factor tables in shared memory.  What crosses CTAs goes
-// through distributed shared memory, each behind one cluster barrier:
-//   * the stencil halo: the first and last rows of the neighbouring CTAs;
-//   * the forward recurrence's carry: each CTA scans its chunks as in the
-//     single-CTA kernel, publishes its total transfer (y_end = a y_start +
-//     b), and folds the totals of the CTAs before it to get its y_start;
-//   * the backward recurrence's carry, likewise from the CTAs after it.
-// Every chunk's carry-in is then ex.a * start + ex.b (ex: the in-CTA
-// exclusive scan), the single-CTA fix-up with a nonzero CTA start.
-template <int M, int P>
-__device__ __forceinline__ void const_solve_cluster(double2 (&r)[M], const double2 *__restrict__ g,
-                                                    const double2 *__restrict__ h, int c,
-                                                    Affine *scratch, Affine *tot_fwd,
-                                                    Affine *tot_bwd, cg::cluster_group &cluster,
-                                                    int rank, int K) {
-  double2 pr[M];
-  double2 y = cmul(g[cslot<M, P>(c, 0)], r[0]);
-  pr[0] = h[cslot<M, P>(c, 0)];
-  r[0] = y;
-#pragma unroll
-  for (int m = 1; m < M; ++m) {
-    const int k = cslot<M, P>(c, m);
-    const double2 hm = h[k];
-    y = cfma(hm, y, cmul(g[k], r[m]));
-    pr[m] = cmul(hm, pr[m - 1]);
-    r[m] = y;
-  }
-  const Affine own_f{pr[M - 1], y};
-  Affine ex = exclusive_scan<P, false>(own_f, scratch);
-  if (c == P - 1) *tot_fwd = compose(ex, own_f);  // this CTA's total transfer
-  cluster.sync();
-  double2 start = mk(0.0, 0.0);  // y at the end of the previous CTA's rows
-  for (int j = 0; j < rank; ++j) {
-    const Affine t = *cluster.map_shared_rank(tot_fwd, j);
-    start = cfma(t.a, start, t.b);
-  }
-  const double2 y_in = cfma(ex.a, start, ex.b);
-#pragma unroll
-  for (int m = 0; m < M; ++m) r[m] = cfma(pr[m], y_in, r[m]);
-  double2 x = r[M - 1];
-  pr[M - 1] = h[cslot<M, P>(c, M - 1)];
-#pragma unroll
-  for (int m = M - 2; m >= 0; --m) {
-    const double2 hm = h[cslot<M, P>(c, m)];
-    x = cfma(hm, x, r[m]);
-    pr[m] = cmul(hm, pr[m + 1]);
-    r[m] = x;
-  }
-  const Affine own_b{pr[0], x};
-  ex = exclusive_scan<P, true>(own_b, scratch);
-  if (c == 0) *tot_bwd = compose(ex, own_b);
-  cluster.sync();
-  start = mk(0.0, 0.0);  // x at the first row of the next CTA
-  for (int j = K - 1; j > rank; --j) {
-    const Affine t = *cluster.map_shared_rank(tot_bwd, j);
-    start = cfma(t.a, start, t.b);
-  }
-  const double2 x_in = cfma(ex.a, start, ex.b);
-#pragma unroll
-  for (int m = 0; m < M; ++m) r[m] = cfma(pr[m], x_in, r[m]);
-}
-
-template <typename R, int M, int T, int K, bool FLUX>
-__global__ void __launch_bounds__(T) cn_const_cluster_kernel(const CnJob *__restrict__ jobs,
-                                                            int step0_ov, int nsteps_ov) {
-  using C = typename Cx<R>::T;
-  constexpr int NC = M * T;  // rows of this CTA
-  cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2 *gs = reinterpret_cast<double2 *>(smem_raw);
-  double2 *hs = gs + NC;
-  double2 *ds = hs + NC;
-  double2 *xch = ds + NC;  // 2 per thread
-  Affine *scratch = reinterpret_cast<Affine *>(xch + 2 * T);
-  __shared__ Affine tot_fwd, tot_bwd;
+  double2 *sL = reinterpret_cast<double2 *>(smem_raw);  // row m of chunk t at m*T + t
+  double2 *sR = sL + NC;
+  double2 *sW = sR + NC;
+  double2 *tot = sW + NC;  // 2 x 2 x TW
   __shared__ double flux_red[2][flux_slots<T>()];
   __shared__ double flux_part[K];
   CnJob job = jobs[blockIdx.x / K];
@@ -363,85 +419,69 @@ __global__ void __launch_bounds__(T) cn_const_cluster_kernel(const CnJob *__rest
     job.step0 = step0_ov;
     job.nsteps = nsteps_ov;
   }
-  const int t = threadIdx.x;
-  const double rho = job.rho, r = job.r;
-  const double2 *gt = reinterpret_cast<const double2 *>(job.lu_g);
-  const double2 *ht = reinterpret_cast<const double2 *>(job.lu_h);
-  const double q = __dmul_rn(0.25, rho);
-  const int base = rank * NC;     // first row of this CTA
-  const int s0 = base + t * M;    // first row of this thread
+  const int t = threadIdx.x, rank = K > 1 ? (int)(blockIdx.x % K) : 0;
+  const int gw = rank * W + t / 32;
+  const int s0 = (rank * T + t) * M;
+  // rows nreal .. pad the system (diagonal kCnPad in the tables, zero field)
   const int nreal = job.n_real > 0 ? job.n_real : K * NC;
+  const double2 *gL = reinterpret_cast<const double2 *>(job.lu_l) + s0;
+  const double2 *gR = reinterpret_cast<const double2 *>(job.lu_r) + s0;
+  const double2 *gW = reinterpret_cast<const double2 *>(job.lu_w) + s0;
+  double2 aL = mk(1.0, 0.0), aR = mk(1.0, 0.0);
 #pragma unroll
   for (int m = 0; m < M; ++m) {
-    const int k = cslot<M, T>(t, m);
-    gs[k] = gt[s0 + m];
-    hs[k] = ht[s0 + m];
-    if (s0 + m < nreal) {
-      const double bp = job.beta_prev[s0 + m], dp = job.delta_prev[s0 + m];
-      const double2 hh = mk(__dmul_rn(0.5, __dmul_rn(bp, r)), __dmul_rn(0.5, __dmul_rn(dp, r)));
-      ds[k] = mk(__dadd_rn(-hh.x, 1.0), __dsub_rn(-hh.y, 0.5 * rho));
-    } else {
-      ds[k] = mk(0.0, 0.0);
-    }
+    sL[m * T + t] = gL[m];
+    sR[m * T + t] = gR[m];
+    sW[m * T + t] = gW[m];
+    aL = cmul(aL, gL[m]);
+    aR = cmul(aR, gR[m]);
   }
   C *field = reinterpret_cast<C *>(job.field);
   double2 u[M];
 #pragma unroll
   for (int m = 0; m < M; ++m) u[m] = s0 + m < nreal ? to_d(field[s0 + m]) : mk(0.0, 0.0);
-  C *saves = reinterpret_cast<C *>(job.saves);
-  const double2 *xch_prev = rank > 0 ? cluster.map_shared_rank(xch, rank - 1) : nullptr;
-  const double2 *xch_next = rank < K - 1 ? cluster.map_shared_rank(xch, rank + 1) : nullptr;
-  for (int st = 0; st < job.nsteps; ++st) {
+  int par = 0;
+  auto publish = [&](int w, int dir, double2 v) {
+    double2 *dst = tot + par * 2 * TW + dir * TW + w;
+    if constexpr (K == 1) {
+      *dst = v;
+    } else {
+#pragma unroll
+      for (int k = 0; k < K; ++k) *cg::this_cluster().map_shared_rank(dst, k) = v;
+    }
+  };
+  auto sync = [] {
+    if constexpr (K == 1) __syncthreads();
+    else cg::this_cluster().sync();
+  };
+  if constexpr (K > 1) cg::this_cluster().sync();  // the peers run: their memory may be written
+  const ScanCoef c = scan_coef<TW>(aL, aR, tot, gw, publish, sync);
+  par = 1;
+  for (int st = 0; st < job.nsteps; ++st, par ^= 1) {
     const int step = job.step0 + st;
     int2 fw;
     const bool flux = FLUX && flux_window(job.flux, step, fw);
-    xch[2 * t] = u[0];
-    xch[2 * t + 1] = u[M - 1];
-    cluster.sync();  // every CTA's edge rows are published
-    double2 lft = mk(0.0, 0.0), rgt = mk(0.0, 0.0);
-    if (t > 0) lft = xch[2 * t - 1];
-    else if (rank > 0) lft = xch_prev[2 * T - 1];
-    if (t < T - 1) rgt = xch[2 * t + 2];
-    else if (rank < K - 1) rgt = xch_next[0];
-    double2 rh[M];
+    double2 x[M];
 #pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const double2 left = m > 0 ? u[m - 1] : lft;
-      const double2 right = s0 + m + 1 >= nreal ? mk(0.0, 0.0) : (m < M - 1 ? u[m + 1] : rgt);
-      const double2 sum = cadd(left, right);
-      rh[m] = s0 + m < nreal ? cfma(ds[cslot<M, T>(t, m)], u[m], mk(-q * sum.y, q * sum.x))
-                             : mk(0.0, 0.0);
-    }
-    const_solve_cluster<M, T>(rh, gs, hs, t, scratch, &tot_fwd, &tot_bwd, cluster, rank, K);
-    const bool save = job.save_every > 0 && saves != nullptr && (step % job.save_every) == 0 &&
-                      (step / job.save_every - 1) < job.max_slots;
-    C *slot = save ? saves + (long long)(step / job.save_every - 1) * nreal : nullptr;
-    double acc = 0.0;
+    for (int m = 0; m < M; ++m) x[m] = u[m];
+    if (job.two_planes) {
+      // (2 + m - m') u, the 2 being in the tables
 #pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const C v = from_d<R>(rh[m]);
-      u[m] = to_d(v);
-      if (save && s0 + m < nreal) slot[s0 + m] = v;
-      if (flux) flux_add(acc, s0 + m, fw, u[m]);
+      for (int m = 0; m < M; ++m)
+        if (s0 + m < nreal) {
+          const double2 h = mk(0.25 * job.r * (job.beta[s0 + m] - job.beta_prev[s0 + m]),
+                               0.25 * job.r * (job.delta[s0 + m] - job.delta_prev[s0 + m]));
+          x[m] = cfma(h, u[m], u[m]);
+        }
     }
-    if constexpr (FLUX) {
-      if (flux) flux_warp_total<T>(acc, flux_red[st & 1]);
-      __syncthreads();
-      if (flux && t < 32) {
-        double v = t < flux_slots<T>() ? flux_red[st & 1][t] : 0.0;
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
-        if (t == 0) *cluster.map_shared_rank(&flux_part[rank], 0) = v;
-      }
-      cluster.sync();  // every CTA's total is in CTA 0's flux_part
-      if (flux && rank == 0 && t == 0) {
-        double v = 0.0;
-        for (int j = 0; j < K; ++j) v += flux_part[j];
-        job.flux.out[step - job.flux.step0] = v;
-      }
-    }
+    two_sided_solve<M, TW>(
+        x, [&](int m) { return sL[m * T + t]; }, [&](int m) { return sR[m * T + t]; },
+        [&](int m) { return sW[m * T + t]; }, c, tot + par * 2 * TW, gw, publish, sync);
+    const double acc = cn_finish<R>(job, step, u, x, s0, nreal, flux, fw);
+    if constexpr (FLUX)
+      if (flux) cn_flux<T, K>(job, step, acc, flux_red, flux_part, rank);
   }
-  cluster.sync();  // no CTA leaves while a peer may still address its shared memory
+  if constexpr (K > 1) cg::this_cluster().sync();  // no CTA leaves while a peer writes to it
 #pragma unroll
   for (int m = 0; m < M; ++m)
     if (s0 + m < nreal) field[s0 + m] = from_d<R>(u[m]);
@@ -449,100 +489,67 @@ __global__ void __launch_bounds__(T) cn_const_cluster_kernel(const CnJob *__rest
 
 static constexpr int kCnM = 8;
 
-template <typename R, int M, int T, bool FLUX>
-static cudaError_t cn_const_launch_f(const CnJob *d_jobs, int nj, int step0, int nsteps,
-                                     cudaStream_t s) {
-  constexpr int N = M * T;
-  constexpr size_t smem = sizeof(double2) * (3 * N + 2 * T) + sizeof(Affine) * (T / 32 + 1);
-  auto k = cn_const_kernel<R, M, T, FLUX>;
-  {  // the static flux slots count against the 48 KB default too
-    const cudaError_t attr = raise_dynamic_smem((const void *)k, (int)smem);
-    if (attr != cudaSuccess) return attr;
-  }
-  k<<<nj, T, smem, s>>>(d_jobs, step0, nsteps);
-  return cudaGetLastError();
-}
-
-template <typename R, int M, int T>
-static cudaError_t cn_const_launch_t(const CnJob *d_jobs, int nj, int step0, int nsteps,
-                                     cudaStream_t s, bool flux) {
-  return flux ? cn_const_launch_f<R, M, T, true>(d_jobs, nj, step0, nsteps, s)
-              : cn_const_launch_f<R, M, T, false>(d_jobs, nj, step0, nsteps, s);
-}
-
-template <typename R, int M, int T, int K, bool FLUX>
-static cudaError_t cn_cluster_launch_f(const CnJob *d_jobs, int nj, int step0, int nsteps,
-                                       cudaStream_t s) {
-  constexpr int NC = M * T;
-  constexpr size_t smem = sizeof(double2) * (3 * NC + 2 * T) + sizeof(Affine) * (T / 32 + 1);
-  auto k = cn_const_cluster_kernel<R, M, T, K, FLUX>;
-  {
-    const cudaError_t attr = raise_dynamic_smem((const void *)k, (int)smem);
-    if (attr != cudaSuccess) return attr;
-  }
+template <typename K_>
+static cudaError_t cn_cluster_launch(K_ kernel, int ctas, int cluster, int threads, size_t smem,
+                                     cudaStream_t s, const CnJob *jobs, int step0, int nsteps) {
+  const cudaError_t e = raise_dynamic_smem((const void *)kernel, (int)smem);
+  if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(K * nj);
-  cfg.blockDim = dim3(T);
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = K;
+  attr[0].val.clusterDim.x = cluster;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k, d_jobs, step0, nsteps);
+  cfg.numAttrs = cluster > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, jobs, step0, nsteps);
 }
 
-template <typename R, int K, int M = 16, int T = 256>
-static cudaError_t cn_cluster_launch_t(const CnJob *d_jobs, int nj, int step0, int nsteps,
-                                       cudaStream_t s, bool flux) {
-  return flux ? cn_cluster_launch_f<R, M, T, K, true>(d_jobs, nj, step0, nsteps, s)
-              : cn_cluster_launch_f<R, M, T, K, false>(d_jobs, nj, step0, nsteps, s);
+template <typename R, int M, int T, int K>
+static cudaError_t cn_const_launch_t(const CnJob *d_jobs, int nj, int step0, int nsteps,
+                                     cudaStream_t s, bool flux) {
+  constexpr size_t smem = sizeof(double2) * (3 * M * T + 4 * (T / 32) * K);
+  return flux ? cn_cluster_launch(cn_const_kernel<R, M, T, K, true>, nj * K, K, T, smem, s, d_jobs,
+                                  step0, nsteps)
+              : cn_cluster_launch(cn_const_kernel<R, M, T, K, false>, nj * K, K, T, smem, s, d_jobs,
+                                  step0, nsteps);
 }
-
-// 4096 rows on a cluster of two CTAs (2048 rows each) is variant 1: the
-// single-CTA step is bound by one SM's FP64 issue rate (about 36 FP64
-// operations a row) and its scans' latency, the pair halves the first and
-// adds two cluster barriers a step.
-int cn_const_variants(Precision, int n) { return n == 4096 ? 2 : 1; }
 
 bool cn_const_supported(Precision, int n) {
-  return n >= 8 * kCnM && !(n & (n - 1)) && n <= 16384;  // 8192, 16384: clusters of 2, 4
+  return n >= 8 * kCnM && !(n & (n - 1)) && n <= 16384;
 }
 
+// Rows a thread, threads a CTA and CTAs a problem.  From 4096 rows on a
+// problem alone is faster on more SMs (4096: 2.17 us a step on one, 1.72 on
+// two, 1.42 on four; 8192 in FP32: 2.93 on two, 2.09 on four; 16384: 2.79 on
+// four, 2.07 on eight), at more SM time a problem: the wide form runs while
+// every problem of the launch finds its SMs free (kSms of them).  Both forms
+// have the same chunks and warps and give the same bits.  2048 rows gain too
+// little (1.40 on one SM, 1.31 on two).
+constexpr int kSms = 148;
 cudaError_t launch_cn_const(Precision p, const CnJob *d_jobs, int nj, int n, int step0, int nsteps,
-                            cudaStream_t s, bool flux, int variant) {
+                            cudaStream_t s, bool flux) {
   if (nj <= 0) return cudaSuccess;
-  if (n == 8192)
-    return p == kFP64 ? cn_cluster_launch_t<double, 2>(d_jobs, nj, step0, nsteps, s, flux)
-                      : cn_cluster_launch_t<float, 2>(d_jobs, nj, step0, nsteps, s, flux);
-  if (n == 16384)
-    return p == kFP64 ? cn_cluster_launch_t<double, 4>(d_jobs, nj, step0, nsteps, s, flux)
-                      : cn_cluster_launch_t<float, 4>(d_jobs, nj, step0, nsteps, s, flux);
-  // n >= 2048: 16 rows per thread (half the threads of 8 rows: fewer warps
-  // in each scan's barriers and shuffles; measured 4.07 -> 3.08 us per step
-  // at n = 4096)
-  if (n == 4096 && variant == 1)
-    return p == kFP64 ? cn_cluster_launch_t<double, 2, 16, 128>(d_jobs, nj, step0, nsteps, s, flux)
-                      : cn_cluster_launch_t<float, 2, 16, 128>(d_jobs, nj, step0, nsteps, s, flux);
-  if (n == 4096)
-    return p == kFP64 ? cn_const_launch_t<double, 16, 256>(d_jobs, nj, step0, nsteps, s, flux)
-                      : cn_const_launch_t<float, 16, 256>(d_jobs, nj, step0, nsteps, s, flux);
-  if (n == 2048)
-    return p == kFP64 ? cn_const_launch_t<double, 16, 128>(d_jobs, nj, step0, nsteps, s, flux)
-                      : cn_const_launch_t<float, 16, 128>(d_jobs, nj, step0, nsteps, s, flux);
-#define PXP_CC(TT)                                                                     \
-  case TT:                                                                             \
-    return p == kFP64 ? cn_const_launch_t<double, kCnM, TT>(d_jobs, nj, step0, nsteps, s, flux) \
-                      : cn_const_launch_t<float, kCnM, TT>(d_jobs, nj, step0, nsteps, s, flux);
-  switch (n / kCnM) {
-    PXP_CC(8) PXP_CC(16) PXP_CC(32) PXP_CC(64) PXP_CC(128)
-    default:
-      return cudaErrorInvalidValue;
+#define PXP_CT(MM, TT, KK)                                                                \
+  p == kFP64 ? cn_const_launch_t<double, MM, TT, KK>(d_jobs, nj, step0, nsteps, s, flux) \
+             : cn_const_launch_t<float, MM, TT, KK>(d_jobs, nj, step0, nsteps, s, flux)
+  switch (n) {
+    case 64: return PXP_CT(2, 32, 1);
+    case 128: return PXP_CT(4, 32, 1);
+    case 256: return PXP_CT(8, 32, 1);
+    case 512: return PXP_CT(8, 64, 1);
+    case 1024: return PXP_CT(8, 128, 1);
+    case 2048: return PXP_CT(16, 128, 1);
+    case 4096: return nj * 4 <= kSms ? PXP_CT(8, 128, 4) : PXP_CT(8, 256, 2);
+    case 8192: return nj * 4 <= kSms ? PXP_CT(16, 128, 4) : PXP_CT(16, 256, 2);
+    case 16384: return nj * 8 <= kSms ? PXP_CT(16, 128, 8) : PXP_CT(16, 256, 4);
+    default: return cudaErrorInvalidValue;
   }
-#undef PXP_CC
+#undef PXP_CT
 }
 
 template <typename R, int T, bool FLUX>

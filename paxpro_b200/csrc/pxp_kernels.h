@@ -74,11 +74,6 @@ cudaError_t launch_fft1d_r8(Precision p, const Fft1dJob *d_jobs, int nj, int n, 
 bool fft1d_r16_enabled(Precision p, int n);
 cudaError_t launch_fft1d_r16(const Fft1dJob *d_jobs, int nj, int step0, int nsteps, cudaStream_t s,
                              bool flux, unsigned *queue = nullptr);
-// Launch variants of CrankNicholson's step-invariant path, chosen per (device,
-// precision, size) by the tuner in capi.cu: at 4096 rows 0 = one CTA, 1 = a
-// cluster of two CTAs.  Returns how many a size has (1: nothing to choose);
-// variant -1 is the default (one CTA).
-int cn_const_variants(Precision p, int n);
 // queue: a device counter (zero at launch) that makes the power-of-two
 // kernels persistent -- at most one wave of CTAs, each taking its next job
 // from the counter (persistent.cuh); null: one CTA per job.
@@ -133,8 +128,8 @@ struct CnJob {
   int n_real;                  // Nx; rows n_real..n-1 are decoupled padding
   int step0, nsteps, save_every, max_slots, mat_step0;
   int transparent;             // BC_t::TRANSPARENT
-  int status;                  // unused (reserved)
-  const void *lu_g, *lu_h;     // factor tables of the step matrix (const path)
+  int two_planes;              // const path: the planes at z and z - dz differ
+  const void *lu_l, *lu_r, *lu_w;  // tables of the two-sided solve (const path, cn.cu)
   FluxSpec flux;               // per-step flux integrals (out == null: none)
 };
 cudaError_t launch_cn(Precision p, const CnJob *d_jobs, int nj, int n, int step0,
@@ -147,9 +142,10 @@ int cn_padded_n(int n);
 // kernels' rows and in the host's factor tables of the step-invariant path.
 constexpr double kCnPad = 1e30;
 // z-invariant medium and Dirichlet ends: the step matrix never changes; the
-// job's lu_g / lu_h hold its Thomas factor tables (n complex128 each).
+// job's lu_l / lu_r / lu_w hold hL, hR and 2 w of the two-sided solve (n
+// complex128 each, see cn.cu).
 cudaError_t launch_cn_const(Precision p, const CnJob *d_jobs, int nj, int n, int step0,
-                            int nsteps, cudaStream_t s, bool flux = false, int variant = -1);
+                            int nsteps, cudaStream_t s, bool flux = false);
 bool cn_const_supported(Precision p, int n);
 
 // ------------------------------------------------------------- ADI ------
