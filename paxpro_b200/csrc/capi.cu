@@ -1823,13 +1823,21 @@ int pxp_step(pxp_solver h, int nsteps) {
         return h->fail(PXP_ERR_UNSUPPORTED,
                        "CrankNicholson at " + std::to_string(h->nx) +
                            " points runs with a z-invariant medium and Dirichlet ends only");
-      if (cn_uses_const(h))
+      if (cn_uses_const(h)) {
         e = pxp::launch_cn_const(h->prec, (const pxp::CnJob *)h->d_job, 1,
                                  pxp::cn_padded_n((int)h->nx), (int)first, nsteps, h->stream,
                                  h->flux_count > 0);
-      else
-        e = pxp::launch_cn(h->prec, (const pxp::CnJob *)h->d_job, 1, pxp::cn_padded_n((int)h->nx),
-                           (int)first, nsteps, h->stream, h->flux_count > 0);
+        break;
+      }
+      e = cudaErrorMemoryAllocation;
+      if (!h->prob.transparent_bc && pxp::cn_planes_supported(pxp::cn_padded_n((int)h->nx), nsteps))
+        e = pxp::launch_cn_planes(h->prec, (const pxp::CnJob *)h->d_job,
+                                  pxp::cn_padded_n((int)h->nx), (int)first, nsteps, h->stream,
+                                  h->flux_count > 0);
+      if (e == cudaErrorMemoryAllocation)
+        e = pxp::launch_cn(h->prec, (const pxp::CnJob *)h->d_job, 1,
+                           pxp::cn_padded_n((int)h->nx), (int)first, nsteps, h->stream,
+                           h->flux_count > 0);
       break;
     case PXP_ADI: {
       int rc = adi_steps(h, (unsigned)first, nsteps);

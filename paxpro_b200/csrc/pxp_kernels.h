@@ -147,6 +147,13 @@ constexpr double kCnPad = 1e30;
 cudaError_t launch_cn_const(Precision p, const CnJob *d_jobs, int nj, int n, int step0,
                             int nsteps, cudaStream_t s, bool flux = false);
 bool cn_const_supported(Precision p, int n);
+// Media sampled per step, Dirichlet ends: the matrices of a block of steps are
+// factored ahead on all SMs (workspace from the stream's pool).  Worth it from
+// some steps a call on; cudaErrorMemoryAllocation (nothing launched) when the
+// workspace cannot be had: launch_cn then.
+bool cn_planes_supported(int n, int nsteps);
+cudaError_t launch_cn_planes(Precision p, const CnJob *d_job, int n, int step0, int nsteps,
+                             cudaStream_t s, bool flux);
 
 // ------------------------------------------------------------- ADI ------
 struct Sphere {
