@@ -33,9 +33,6 @@
 
 namespace pxp {
 
-// kernel waits that ran out on this device (never reset), read by the host
-__device__ unsigned int g_wait_timeouts = 0;
-
 // The material of the half step's plane at (x, y); idx: the point's index in
 // the field's layout, for a sampled plane.
 __device__ __forceinline__ void sphere_material(const AdiHalf &h, double x, double y,
@@ -777,7 +774,7 @@ __global__ void __launch_bounds__(((G + S - 1) / S) * (N / M), 1)
   if (tid == 0) {
     const bool ok = mbar_wait_bounded(bar, 0, 2000000000ull);
     if (!ok) {
-      atomicAdd(&g_wait_timeouts, 1u);
+      atomicAdd(h.timeouts, 1u);
       mbar_wait_bounded(bar, 0, 2000000000ull);  // the table copy may still be in flight
     }
     staged_ok = ok;
@@ -923,7 +920,7 @@ __global__ void __launch_bounds__(((G + S - 1) / S) * (N / M), 1)
   if (gtid == 0) {
     bool ok = mbar_wait_bounded(bar + 1 + group, 0, 2000000000ull);
     ok = mbar_wait_bounded(bar, 0, 2000000000ull) && ok;
-    if (!ok) atomicAdd(&g_wait_timeouts, 1u);
+    if (!ok) atomicAdd(h.timeouts, 1u);
     group_ok[group] = ok;
   }
   group_sync(1 + group, P);
@@ -1127,25 +1124,16 @@ bool adi_const_staged_tables(int n, const double *g, const double *h, double *ou
 // the kernels' bounded wait (mbar_wait_bounded) and the given limit.  The
 // wait runs out, the kernel records it in the same counter the propagation
 // kernels use, and returns; nothing faults and the context stays usable.
-__global__ void wait_selftest_kernel(unsigned long long limit_ns) {
+__global__ void wait_selftest_kernel(unsigned long long limit_ns, unsigned *timeouts) {
   __shared__ __align__(8) uint64_t bar;
   mbar_init(&bar, 1);
   mbar_arrive_expect_tx(&bar, 16u);
-  if (!mbar_wait_bounded(&bar, 0, limit_ns)) atomicAdd(&g_wait_timeouts, 1u);
+  if (!mbar_wait_bounded(&bar, 0, limit_ns)) atomicAdd(timeouts, 1u);
 }
 
-cudaError_t launch_wait_selftest(unsigned long long limit_ns, cudaStream_t s) {
-  wait_selftest_kernel<<<1, 1, 0, s>>>(limit_ns);
+cudaError_t launch_wait_selftest(unsigned long long limit_ns, unsigned *timeouts, cudaStream_t s) {
+  wait_selftest_kernel<<<1, 1, 0, s>>>(limit_ns, timeouts);
   return cudaGetLastError();
-}
-
-unsigned wait_timeouts(cudaStream_t s) {
-  unsigned v = 0;
-  if (cudaMemcpyFromSymbolAsync(&v, g_wait_timeouts, sizeof(v), 0, cudaMemcpyDeviceToHost, s) !=
-          cudaSuccess ||
-      cudaStreamSynchronize(s) != cudaSuccess)
-    return 0;
-  return v + fft3d_lines_wait_timeouts(s) + fft3d_r16_wait_timeouts(s);
 }
 
 cudaError_t launch_adi_half_const(Precision p, const AdiHalf &h, const void *g, const void *hh,

@@ -110,7 +110,11 @@ struct pxp_solver_s {
   bool material_set = false;
   bool ic_set = false;
   unsigned current_step = 1;
-  unsigned timeouts_seen = 0;  // device count of ran-out kernel waits at creation
+  // the device's count of ran-out kernel waits (wait_counter.cu): the host's
+  // address, the kernels' and the count at creation
+  const volatile unsigned *timeouts = nullptr;
+  unsigned *d_timeouts = nullptr;
+  unsigned timeouts_seen = 0;
   // saved fields: save_pts points each (3-D kinds: save_n x save_n block
   // averages of the field when the transverse downsampling ratio is above 1,
   // staged through d_save_stage)
@@ -864,6 +868,7 @@ int adi_step(pxp_solver_s *h, unsigned step) {
   pxp::AdiHalf a{};
   a.n = (int)n;
   a.use_tbc = p.transparent_bc ? 1 : 0;
+  a.timeouts = h->d_timeouts;
   a.inv_dzh = 1.0 / dzh;
   a.k = k;
   a.xmin = p.x.min;
@@ -1158,6 +1163,7 @@ int fft3d_steps(pxp_solver_s *h, unsigned first, int nsteps) {
   q.chirp = h->d_chirp;
   q.bconv = h->d_bconv;
   q.m = pxp::fft1d_bluestein_m(n);
+  q.timeouts = h->d_timeouts;
   q.n = n;
   q.a = 0.5 * p.z.step / p.wavenumber;  // FFTSolver3D::kernel (src/fftSolver3D.cpp:24-30)
   q.two_pi = 2.0 * PI;
@@ -1416,7 +1422,6 @@ int pxp_solver_create(const pxp_problem *problem, pxp_solver *out) {
     delete h;
     return PXP_ERR_CUDA;
   }
-  h->timeouts_seen = pxp::wait_timeouts(h->stream);
   int rc = PXP_OK;
   auto cleanup_fail = [&](int code) {
     std::string m = h->err;
@@ -1424,6 +1429,9 @@ int pxp_solver_create(const pxp_problem *problem, pxp_solver *out) {
     set_global_error(m);
     return code;
   };
+  h->timeouts = pxp::wait_counter(p.device, &h->d_timeouts);
+  if (h->timeouts == nullptr) return cleanup_fail(h->fail(PXP_ERR_NOMEM, "wait counter allocation"));
+  h->timeouts_seen = *h->timeouts;
   if ((rc = alloc(h, &h->d_field, h->csize * h->npts, "field"))) return cleanup_fail(rc);
   PXP_TRY_CUDA(h, cudaMemset(h->d_field, 0, h->csize * h->npts));
   h->save_every = p.save_every > 0 ? p.save_every : 0;
@@ -1758,25 +1766,27 @@ static int upload_field(pxp_solver_s *h, void *dst, const double *src) {
 }
 
 // A kernel of this device gave up a bounded wait since the handle was made:
-// its results are not to be trusted.
-static int check_waits(pxp_solver_s *h) {
-  if (pxp::wait_timeouts(h->stream) != h->timeouts_seen)
+// its results are not to be trusted.  After a synchronisation of the stream.
+static int waits_held(pxp_solver_s *h) {
+  if (*h->timeouts != h->timeouts_seen)
     return h->fail(PXP_ERR_CUDA, "a kernel's bounded wait for its copies ran out on this device");
   return PXP_OK;
+}
+static int check_waits(pxp_solver_s *h) {
+  PXP_TRY_CUDA(h, cudaStreamSynchronize(h->stream));
+  return waits_held(h);
 }
 
 static int download_field(pxp_solver_s *h, double *dst, const void *src, long long npts = -1) {
   if (npts < 0) npts = h->npts;
-  if (int rc = check_waits(h)) return rc;
   if (h->prec == pxp::kFP64) {
     PXP_TRY_CUDA(h, cudaMemcpyAsync(dst, src, 16 * npts, cudaMemcpyDeviceToHost, h->stream));
-    PXP_TRY_CUDA(h, cudaStreamSynchronize(h->stream));
-  } else {
-    std::vector<float> tmp(2 * npts);
-    PXP_TRY_CUDA(h, cudaMemcpyAsync(tmp.data(), src, 8 * npts, cudaMemcpyDeviceToHost, h->stream));
-    PXP_TRY_CUDA(h, cudaStreamSynchronize(h->stream));
-    for (long long i = 0; i < 2 * npts; ++i) dst[i] = (double)tmp[i];
+    return check_waits(h);
   }
+  std::vector<float> tmp(2 * npts);
+  PXP_TRY_CUDA(h, cudaMemcpyAsync(tmp.data(), src, 8 * npts, cudaMemcpyDeviceToHost, h->stream));
+  if (int rc = check_waits(h)) return rc;
+  for (long long i = 0; i < 2 * npts; ++i) dst[i] = (double)tmp[i];
   return PXP_OK;
 }
 
@@ -1865,13 +1875,12 @@ int pxp_solve(pxp_solver h) {
 
 int pxp_synchronize(pxp_solver h) {
   if (h == nullptr) return PXP_ERR_INVALID;
-  PXP_TRY_CUDA(h, cudaStreamSynchronize(h->stream));
   return check_waits(h);
 }
 
 int pxp_selftest_bounded_wait(pxp_solver h, unsigned long long limit_ns) {
   if (h == nullptr || limit_ns == 0 || limit_ns > 10000000000ull) return PXP_ERR_INVALID;
-  cudaError_t e = pxp::launch_wait_selftest(limit_ns, h->stream);
+  cudaError_t e = pxp::launch_wait_selftest(limit_ns, h->d_timeouts, h->stream);
   if (e != cudaSuccess) return h->cuda_fail(e, "bounded-wait self-test launch");
   return PXP_OK;
 }

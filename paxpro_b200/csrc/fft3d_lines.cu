@@ -53,9 +53,6 @@
 
 namespace pxp {
 
-// waits of these kernels that ran out on this device, read by the host
-__device__ unsigned int g_lines_wait_timeouts = 0;
-
 namespace lines {
 
 __host__ __device__ constexpr int ilog2c(int n) { return n <= 1 ? 0 : 1 + ilog2c(n / 2); }
@@ -301,7 +298,7 @@ __global__ void __launch_bounds__(Cfg<R, N, LG>::T, Cfg<R, N, LG>::MINB)
     if (tid == 0) {
       const bool ok = mbar_wait_bounded(bar, it & 1, 2000000000ull);
       if (!ok) {
-        atomicAdd(&g_lines_wait_timeouts, 1u);
+        atomicAdd(q.timeouts, 1u);
         mbar_wait_bounded(bar, it & 1, 2000000000ull);  // the copy may still be in flight
       }
       s_ok = ok;
@@ -608,15 +605,6 @@ cudaError_t launch_fft3d_lines(Precision p, const Fft3dPass &q, const double *kx
       return cudaErrorInvalidValue;
   }
 #undef PXP_L3
-}
-
-unsigned fft3d_lines_wait_timeouts(cudaStream_t s) {
-  unsigned v = 0;
-  if (cudaMemcpyFromSymbolAsync(&v, g_lines_wait_timeouts, sizeof(v), 0, cudaMemcpyDeviceToHost,
-                                s) != cudaSuccess ||
-      cudaStreamSynchronize(s) != cudaSuccess)
-    return 0;
-  return v;
 }
 
 }  // namespace pxp

@@ -50,10 +50,6 @@
 
 namespace pxp {
 
-// waits of the radix-16 line kernel that ran out on this device, read by
-// the host
-__device__ unsigned int g_r16_wait_timeouts = 0;
-
 cudaError_t encode_field_tmap(void *field, int n, int real_bytes, int box_reals, int box_rows,
                               CUtensorMap *out);
 namespace r16 {
@@ -267,7 +263,7 @@ __global__ void __launch_bounds__(Cfg<R, N, LP, SL>::T, Cfg<R, N, LP, SL>::MINB)
               "l"(&tmap), "r"(2 * line0), "r"(b * K::BOX), "r"(smem_u32(sbar))
               : "memory");
         if (!mbar_wait_bounded(sbar, it & 1, 2000000000ull)) {
-          atomicAdd(&g_r16_wait_timeouts, 1u);
+          atomicAdd(q.timeouts, 1u);
           mbar_wait_bounded(sbar, it & 1, 2000000000ull);  // the copy may still be in flight
           slot_fail[slot] = 1;
         }
@@ -428,15 +424,6 @@ cudaError_t launch(const Fft3dPass &q, const double *kx2, const void *wnv, cudaS
 }
 
 }  // namespace r16
-
-unsigned fft3d_r16_wait_timeouts(cudaStream_t s) {
-  unsigned v = 0;
-  if (cudaMemcpyFromSymbolAsync(&v, g_r16_wait_timeouts, sizeof(v), 0, cudaMemcpyDeviceToHost,
-                                s) != cudaSuccess ||
-      cudaStreamSynchronize(s) != cudaSuccess)
-    return 0;
-  return v;
-}
 
 bool fft3d_r16_supported(Precision p, int n, bool single) {
   if (single && p != kFP32) return false;

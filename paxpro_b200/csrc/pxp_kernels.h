@@ -209,6 +209,7 @@ struct AdiHalf {
   // one-wave vacuum kernel: chunks tab_c0 < c < tab_c1 of the staged tables
   // hold bit for bit the entries of chunk tab_c0 and read those (0, 0: none)
   int tab_c0, tab_c1;
+  unsigned *timeouts;      // counts waits that ran out (one-wave vacuum kernels)
   Csg csg;                 // CSG material (instead of spheres) when csg.active
   // sampled material of this half step's plane (instead of spheres or CSG)
   // when plane_delta is set: n*n doubles each, the field's layout (x index *
@@ -305,12 +306,13 @@ cudaError_t launch_flux_sum(Precision p, const void *field, int a, int b, double
 // complex64 -> complex128, n entries.
 cudaError_t launch_widen(const void *in, void *out, long long n, cudaStream_t s);
 
-// Kernel waits on the current device that ran out (bounded mbarrier waits),
-// read on stream s (synchronises s).
-unsigned wait_timeouts(cudaStream_t s);
+// The word of mapped host memory that counts the kernel waits of `device` that
+// ran out (bounded mbarrier waits, wait_counter.cu): the host's address, *dev
+// (may be null) the device's.  The device must be current.
+unsigned *wait_counter(int device, unsigned **dev);
 // One-thread kernel whose bounded wait (limit_ns of global time) runs out on
 // purpose and is counted like the propagation kernels' (adi.cu).
-cudaError_t launch_wait_selftest(unsigned long long limit_ns, cudaStream_t s);
+cudaError_t launch_wait_selftest(unsigned long long limit_ns, unsigned *timeouts, cudaStream_t s);
 
 // --------------------------------------------------------------- FFT 3-D --
 // FFTSolver3D (src/fftSolver3D.cpp:52-156, 327-374) on an n x n field in the
@@ -365,6 +367,7 @@ struct Fft3dPass {
   // (fft3d_lines.cu, n = 1024 .. 4096): entry i = exp(-2 pi i m_i / n), m_i from
   // fft3d_lines_tw_exponents, in the solver's table form
   const void *tw_lines;
+  unsigned *timeouts;      // counts waits that ran out
 };
 // Exponents m_i of the twiddle table Fft3dPass::tw_lines for length n (out:
 // room for cap entries); returns the entry count (0: the kernel for n reads
@@ -398,8 +401,5 @@ cudaError_t launch_fft3d_bluestein(Precision p, const Fft3dPass &q, const double
 cudaError_t launch_fft3d_mixed(Precision p, const Fft3dPass &q, const double *kx2, cudaStream_t s);
 cudaError_t launch_fft3d_lines(Precision p, const Fft3dPass &q, const double *kx2, const void *wn,
                                cudaStream_t s);
-// Bounded waits of the line-pass kernels that ran out on the current device.
-unsigned fft3d_lines_wait_timeouts(cudaStream_t s);
-unsigned fft3d_r16_wait_timeouts(cudaStream_t s);
 
 }  // namespace pxp
