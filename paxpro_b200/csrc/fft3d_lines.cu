@@ -94,12 +94,25 @@ template <typename R, int N, int LG> struct Cfg {
   static constexpr size_t STAGE = sizeof(C) * (size_t)L * N;
   static constexpr size_t XBYTES = sizeof(C) * (size_t)L * XS;
   static constexpr size_t SMEM = 128 + STAGE + 2 * ((XBYTES + 127) & ~size_t(127)) + 128;
+  // Complex64: one copy of the transform's code serves both directions (the
+  // inverse is the forward transform of the swapped (im, re) values, swapped
+  // back by the pointwise work around it).  With a copy for each the code of a
+  // group of two lines a thread outgrows the instruction cache (some 2200
+  // instructions; 1.7 of 5.9 cycles an instruction waited for it in the y
+  // pass).  us a step: 512 11.1 -> 9.2, 1024 26.0 -> 25.1, 2048 81.4 -> 79.7.
+  // Complex128 lines, one a thread, have half the code, and the buffers'
+  // addresses, known at compile time with two copies, count (4096: 483 -> 510
+  // with one, 256: 7.6 -> 7.8).
+  static constexpr bool ONE_DIR = sizeof(R) == 4;
   static_assert(N % 8 == 0 && T <= 1024, "line slots");
 };
 
 template <typename C, typename W> __device__ __forceinline__ C twm(C v, W w, bool fwd) {
   return fwd ? tw_mul(v, w) : tw_mulc(v, w);
 }
+
+__device__ __forceinline__ double2 swapri(double2 a) { return mk(a.y, a.x); }
+__device__ __forceinline__ float2 swapri(float2 a) { return mk(a.y, a.x); }
 
 // First pass (NS = 1, radix R0) on the thread's 8 points j + s*n/8, result
 // to exchange buffer X at the Stockham positions b*R0 + r of its butterflies
@@ -318,6 +331,7 @@ __global__ void __launch_bounds__(Cfg<R, N, LG>::T, Cfg<R, N, LG>::MINB)
       for (int s = 0; s < 8; ++s) {
         const int e = j + s * K::TL;
         v[t][s] = xpass ? S[e * K::L + l] : S[l * N + e];
+        if (K::ONE_DIR && q.mode >= 2) v[t][s] = swapri(v[t][s]);
       }
     }
     // The staging buffer is free once every thread has read it, which the
@@ -330,27 +344,15 @@ __global__ void __launch_bounds__(Cfg<R, N, LG>::T, Cfg<R, N, LG>::MINB)
     };
     auto nothing = [] {};
 
-    if (q.mode == 1) {
-      line_fft<-1, R, N, LG>(v, X0, X1, cur, tw, tws, slot, j, issue_next);
-      // propagator K = exp(-i a (kx^2 + ky^2)) (src/fftSolver3D.cpp:24-30, 87-120)
-#pragma unroll
-      for (int t = 0; t < K::LPT; ++t) {
-        const int line = line0 + slot * K::LPT + t;  // y index
-        const double ky = kfreq(line, N, q.two_pi, q.stepn_y);
-        const double ky2 = __dmul_rn(ky, ky);
-#pragma unroll
-        for (int s = 0; s < 8; ++s) v[t][s] = prop3(q, v[t][s], kx2[s], ky2, j + s * K::TL, line);
-      }
-      line_fft<+1, R, N, LG>(v, X0, X1, cur, tw, tws, slot, j, nothing);
-    } else if (q.mode == 0) {
-      line_fft<-1, R, N, LG>(v, X0, X1, cur, tw, tws, slot, j, issue_next);
-    } else {
-      line_fft<+1, R, N, LG>(v, X0, X1, cur, tw, tws, slot, j, issue_next);
+    // The refraction between a y pass's transforms: the inverse transform's
+    // points (swapped when ONE_DIR) in v become the refracted ones.
+    auto unswap = [](C a) { return K::ONE_DIR ? swapri(a) : a; };
+    auto refract_points = [&] {
       if (scale_only) {
 #pragma unroll
         for (int t = 0; t < K::LPT; ++t)
 #pragma unroll
-          for (int s = 0; s < 8; ++s) v[t][s] = scale_point(v[t][s], inv_norm);
+          for (int s = 0; s < 8; ++s) v[t][s] = scale_point(unswap(v[t][s]), inv_norm);
       } else {
         // material or absorber in this step: the thread's own points go
         // through the exchange buffer the last pass did not read (every
@@ -361,7 +363,7 @@ __global__ void __launch_bounds__(Cfg<R, N, LG>::T, Cfg<R, N, LG>::MINB)
 #pragma unroll
         for (int t = 0; t < K::LPT; ++t)
 #pragma unroll
-          for (int s = 0; s < 8; ++s) scr[t * K::XS + j + s * K::TL] = v[t][s];
+          for (int s = 0; s < 8; ++s) scr[t * K::XS + j + s * K::TL] = unswap(v[t][s]);
 #pragma unroll 1
         for (int i = 0; i < 8 * K::LPT; ++i) {
           const int t = i / 8, e = j + (i % 8) * K::TL;  // e: y index
@@ -381,6 +383,42 @@ __global__ void __launch_bounds__(Cfg<R, N, LG>::T, Cfg<R, N, LG>::MINB)
           for (int s = 0; s < 8; ++s)
             save[(long long)(line0 + slot * K::LPT + t) * N + j + s * K::TL] = v[t][s];
       }
+    };
+    // propagator K = exp(-i a (kx^2 + ky^2)) (src/fftSolver3D.cpp:24-30, 87-120)
+    auto propagate_points = [&] {
+#pragma unroll
+      for (int t = 0; t < K::LPT; ++t) {
+        const int line = line0 + slot * K::LPT + t;  // y index
+        const double ky = kfreq(line, N, q.two_pi, q.stepn_y);
+        const double ky2 = __dmul_rn(ky, ky);
+#pragma unroll
+        for (int s = 0; s < 8; ++s)
+          v[t][s] = unswap(prop3(q, v[t][s], kx2[s], ky2, j + s * K::TL, line));
+      }
+    };
+
+    if constexpr (K::ONE_DIR) {
+      // mode 1: forward, propagator, inverse; mode 2: inverse, refraction,
+      // forward; mode 0: forward; mode 3: inverse, refraction
+      const int transforms = q.mode == 1 || q.mode == 2 ? 2 : 1;
+#pragma unroll 1
+      for (int ph = 0; ph < transforms; ++ph) {
+        line_fft<-1, R, N, LG>(v, X0, X1, cur, tw, tws, slot, j, [&] {
+          if (ph == 0) issue_next();
+        });
+        if (ph > 0) break;
+        if (q.mode == 1) propagate_points();
+        if (q.mode >= 2) refract_points();
+      }
+    } else if (q.mode == 1) {
+      line_fft<-1, R, N, LG>(v, X0, X1, cur, tw, tws, slot, j, issue_next);
+      propagate_points();
+      line_fft<+1, R, N, LG>(v, X0, X1, cur, tw, tws, slot, j, nothing);
+    } else if (q.mode == 0) {
+      line_fft<-1, R, N, LG>(v, X0, X1, cur, tw, tws, slot, j, issue_next);
+    } else {
+      line_fft<+1, R, N, LG>(v, X0, X1, cur, tw, tws, slot, j, issue_next);
+      refract_points();
       if (q.mode != 3) line_fft<-1, R, N, LG>(v, X0, X1, cur, tw, tws, slot, j, nothing);
     }
     if (xpass && K::WARP_ST) {
@@ -393,7 +431,7 @@ __global__ void __launch_bounds__(Cfg<R, N, LG>::T, Cfg<R, N, LG>::MINB)
       const int lane = tid & 31, w0 = tid & ~31;
       __syncwarp();
 #pragma unroll
-      for (int s = 0; s < 8; ++s) F[j + s * K::TL] = v[0][s];
+      for (int s = 0; s < 8; ++s) F[j + s * K::TL] = K::ONE_DIR ? swapri(v[0][s]) : v[0][s];
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       __syncwarp();
       if (lane == 0) {
@@ -421,7 +459,8 @@ __global__ void __launch_bounds__(Cfg<R, N, LG>::T, Cfg<R, N, LG>::MINB)
 #pragma unroll
       for (int t = 0; t < K::LPT; ++t)
 #pragma unroll
-        for (int s = 0; s < 8; ++s) F[(j + s * K::TL) * K::L + slot * K::LPT + t] = v[t][s];
+        for (int s = 0; s < 8; ++s)
+          F[(j + s * K::TL) * K::L + slot * K::LPT + t] = K::ONE_DIR ? swapri(v[t][s]) : v[t][s];
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       __syncthreads();
       if (tid == 0) {
