@@ -1147,9 +1147,21 @@ cudaError_t launch_adi_half_const(Precision p, const AdiHalf &h, const void *g, 
       case 64: return adi_const_wave_launch<64, 2, 4, 2>(h, staged, s);
       case 128: return adi_const_wave_launch<128, 4, 2, 1>(h, staged, s);
       case 256: return adi_const_wave_launch<256, 8, 2, 1>(h, staged, s);
-      case 512: return adi_const_wave_launch<512, 8, 4, 2>(h, staged, s);
-      case 768: return adi_const_wave_launch<768, 8, 6, 2>(h, staged, s);
-      case 1024: return adi_const_wave_launch<1024, 8, 7, 2>(h, staged, s);
+      // systems a CTA: as few as still make one wave of the 148 SMs (us a step:
+      // 290 nodes 9.7 with four, 7.2 with two; 513 16.0 with six, 12.9 with
+      // four; 800 23.0 with seven, 19.2 with six); three at 297 .. 444 nodes,
+      // a full group of two and a half empty one, are slower than four (440:
+      // 12.1 against 11.2)
+      case 512:
+        if (h.n <= 296) return adi_const_wave_launch<512, 8, 2, 1>(h, staged, s);
+        return adi_const_wave_launch<512, 8, 4, 2>(h, staged, s);
+      case 768:
+        if (h.n <= 592) return adi_const_wave_launch<768, 8, 4, 2>(h, staged, s);
+        if (h.n <= 740) return adi_const_wave_launch<768, 8, 5, 2>(h, staged, s);
+        return adi_const_wave_launch<768, 8, 6, 2>(h, staged, s);
+      case 1024:
+        if (h.n <= 888) return adi_const_wave_launch<1024, 8, 6, 2>(h, staged, s);
+        return adi_const_wave_launch<1024, 8, 7, 2>(h, staged, s);
       default: break;
     }
   }

@@ -30,3 +30,14 @@ def test_general_half_step_at_launch_shape_edges(n, use_tbc, precision):
             assert _rel(a, b) <= FP64_TOL
         else:
             assert _int_rel(a, b) <= FP32_INT_TOL
+
+
+@pytest.mark.parametrize("n", [257, 296, 297, 513, 592, 593, 740, 741, 769, 888, 889])
+def test_vacuum_half_step_at_launch_shape_edges(n):
+    """The one-wave vacuum kernel where its systems a CTA change."""
+    x = -500.0 + wl.step_for_nodes(-500.0, 500.0, n) * np.arange(n)
+    g = np.exp(-((x - 40.0) / 300.0) ** 2) * np.exp(1j * 2e-3 * x)
+    u0 = np.asfortranarray(g[:, None] * g[None, :])
+    out, saves, ref_out, ref_saves = _run_both(n, 0.0, 4, 1000.0, [], u0=u0)
+    assert len(saves) == len(ref_saves) == 4
+    assert max(_rel(a, b) for a, b in zip(saves, ref_saves)) <= FP64_TOL
