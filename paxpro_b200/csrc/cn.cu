@@ -1,11 +1,15 @@
-// cn.cu -- K-CN: Crank-Nicolson step with a fused tridiagonal solve.
+// cn.cu -- K-CN: Crank-Nicolson steps.
 //
 // Replaces CrankNicholson::solveStep (src/crancNicholson.cpp:17-105) with the
 // default ParaxialEquation (F = G = H = 1, J = 0, src/paraxialEquation.cpp:
-// 3-21) and ThomasAlgorithm::solve (include/thomasAlgorithm.tpp:2-32).
-//
-// One CTA owns one problem; the field stays in shared memory for every step
-// of the launch.  Per step:
+// 3-21) and ThomasAlgorithm::solve (include/thomasAlgorithm.tpp:2-32).  A CTA
+// (or a cluster) owns one problem; the field stays on chip for every step of
+// the launch.  Three kernels:
+//   cn_const_kernel   z-invariant media, Dirichlet ends;
+//   cn_planes_kernel  media sampled per step, Dirichlet ends, a block of steps
+//                     factored ahead by cn_factor_kernel;
+//   cn_kernel         everything else (transparent ends, short calls, batches
+//                     of sampled media), step by step:
 //   1. each thread builds the matrix rows of its chunk of M consecutive points
 //      (diag, rhs; sub-diagonal constant) with the reference's operation
 //      order, rounded op by op, so the coefficients equal the reference's;
@@ -15,11 +19,11 @@
 //      unknowns;
 //   3. the CTA solves the reduced system by cyclic reduction in shared memory;
 //   4. each thread reconstructs its interior.
-// The solve runs in FP64 in both storage precisions: with rho = dz/(k dx^2)
-// of a few hundred the system is only weakly diagonally dominant.
-// The split into chunks changes the rounding relative to the reference's
-// serial Thomas sweep; the step matrix is well conditioned (Cayley transform,
-// condition ~ rho), so the difference stays near machine precision.
+// The solves run in FP64 in both storage precisions: with rho = dz/(k dx^2)
+// of a few hundred the system is only weakly diagonally dominant.  They differ
+// from the reference's serial Thomas sweep in rounding; the step matrix is
+// well conditioned (Cayley transform, condition ~ rho), so the difference
+// stays near machine precision.
 #include "pxp_complex.cuh"
 #include "flux.cuh"
 #include "pxp_kernels.h"

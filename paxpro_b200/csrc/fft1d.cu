@@ -1,11 +1,16 @@
-// fft1d.cu -- K-FFT1: fused split-step kernel for one transverse dimension.
+// fft1d.cu -- K-FFT1: fused split-step kernels for one transverse dimension
+// whose field lives in shared memory, and the choice of the kernel for a length.
 //
 // Replaces FFTSolver2D::solveStep (src/fftSolver2D.cpp:61-73): forward FFT,
 // propagator multiply (:21-34), backward FFT, transmission multiply and 1/N
-// normalisation (:36-50).  One CTA owns one problem and keeps its field in
-// shared memory for all steps of the launch, so HBM sees the field once per
-// launch plus the save slots; the only per-step global reads are the
-// propagator and transmission tables, which stay in L2.
+// normalisation (:36-50).  One CTA owns one problem and keeps its field on
+// chip for all steps of the launch, so HBM sees the field once per launch plus
+// the save slots; the only per-step global reads are the propagator and
+// transmission tables, which stay in L2.  Powers of two from 64 to 4096 points
+// keep the field in registers (fft1d_r8.cu, fft1d_r16.cu), complex128 lines of
+// 16384 run on two CTAs (fft1d_pair.cu), lengths with prime factors up to 31
+// mixed-radix (fft1d_mixed.cu); here are the other powers of two and
+// Bluestein's transform for the other lengths.
 //
 // FP64 mode reproduces the reference's pointwise arithmetic exactly:
 // curr *= kernel is a rounded complex product and the refraction update is

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "mixed_plan.h"
+
 namespace pxp {
 
 enum Precision { kFP64 = 0, kFP32 = 1 };
@@ -91,26 +93,7 @@ inline bool fft1d_pair_size(Precision p, int n) { return p == kFP64 && n == 1638
 // smallest power of two >= 2n - 1); n itself for powers of two.
 int fft1d_bluestein_m(int n);
 
-// Passes of the mixed-radix transform (fft_mixed.cuh) of length n, in order:
-// radix, butterflies (n / radix), the multiplier that divides a butterfly's
-// index by the pass's sub-transform length, and for radices above 9 where
-// their (cos, sin) factors lie in the table (16 bytes: one load a pass).
-struct MixedPlan {
-  static constexpr int kMaxPasses = 8;
-  struct alignas(16) Pass {
-    int radix, nb;
-    unsigned magic;
-    int rot;
-  };
-  Pass pass[kMaxPasses];
-  int n, passes;
-  int table;  // entries of the table
-  bool big;   // a radix above 13
-};
-// Fills *plan (may be null) and returns true for lengths that are not powers
-// of two and have no prime factor above 31.
-bool mixed_plan(int n, MixedPlan *plan);
-// FFTSolver2D steps of such lengths (fft1d_mixed.cu); the job's twiddle is the
+// FFTSolver2D steps of the lengths that mixed_plan takes (fft1d_mixed.cu); the job's twiddle is the
 // plan's table.
 cudaError_t launch_fft1d_mixed(Precision p, const Fft1dJob *d_jobs, int nj, int n, int step0,
                                int nsteps, cudaStream_t s, bool flux);

@@ -1,9 +1,8 @@
 // scan_solve.cuh -- tridiagonal solve with a step-invariant matrix as two
 // parallel linear-recurrence scans.
 //
-// When the system matrix does not change between steps (CrankNicholson with a
-// z-invariant medium and Dirichlet ends; an ADI half step whose plane holds
-// no material), its Thomas factorisation (include/thomasAlgorithm.tpp:2-32)
+// When the system matrix does not change between steps (an ADI half step whose
+// plane holds no material), its Thomas factorisation (include/thomasAlgorithm.tpp:2-32)
 // is computed once on the host:
 //   den_0 = b_0,  den_i = b_i - s * c'_{i-1},  c'_i = s / den_i,
 // and stored per position as g_i = 1/den_i and h_i = -s * g_i (s = the
@@ -179,83 +178,6 @@ __host__ __device__ __forceinline__ int cslot(int c, int m) {
 template <int M, int P>
 __host__ __device__ __forceinline__ int cslot_pos(int p) {
   return cslot<M, P>(p / M, p % M);
-}
-
-// const_solve with the factor tables in chunk-transposed slots (cslot) and
-// the step-invariant in-chunk products of the multipliers read from tables:
-// pf at a row holds the product of h over the chunk's rows up to and
-// including it (forward), pb over the rows from it to the chunk's end
-// (backward).  Same recurrences and scans as const_solve.
-template <int M, int P>
-__device__ __forceinline__ void const_solve_tab(double2 (&r)[M], const double2 *__restrict__ g,
-                                                const double2 *__restrict__ h,
-                                                const double2 *__restrict__ pf,
-                                                const double2 *__restrict__ pb, int c,
-                                                Affine *scratch) {
-  // forward, zero carry-in: y_i = g_i r_i + h_i y_{i-1}
-  double2 y = cmul(g[cslot<M, P>(c, 0)], r[0]);
-  r[0] = y;
-#pragma unroll
-  for (int m = 1; m < M; ++m) {
-    const int k = cslot<M, P>(c, m);
-    y = cfma(h[k], y, cmul(g[k], r[m]));
-    r[m] = y;
-  }
-  Affine ex = exclusive_scan<P, false>(Affine{pf[cslot<M, P>(c, M - 1)], y}, scratch);
-  const double2 y_in = ex.b;
-#pragma unroll
-  for (int m = 0; m < M; ++m) r[m] = cfma(pf[cslot<M, P>(c, m)], y_in, r[m]);
-  // backward, zero carry-in: x_i = y_i + h_i x_{i+1}
-  double2 x = r[M - 1];
-#pragma unroll
-  for (int m = M - 2; m >= 0; --m) {
-    x = cfma(h[cslot<M, P>(c, m)], x, r[m]);
-    r[m] = x;
-  }
-  ex = exclusive_scan<P, true>(Affine{pb[cslot<M, P>(c, 0)], x}, scratch);
-  const double2 x_in = ex.b;
-#pragma unroll
-  for (int m = 0; m < M; ++m) r[m] = cfma(pb[cslot<M, P>(c, m)], x_in, r[m]);
-}
-
-// const_solve with the factor tables in chunk-transposed slots (cslot) and
-// the in-chunk products of the multipliers formed in the sweeps and kept in
-// registers for the carry-in fix-ups.
-template <int M, int P>
-__device__ __forceinline__ void const_solve_reg(double2 (&r)[M], const double2 *__restrict__ g,
-                                                const double2 *__restrict__ h, int c,
-                                                Affine *scratch) {
-  double2 pr[M];
-  // forward, zero carry-in: y_i = g_i r_i + h_i y_{i-1}
-  double2 y = cmul(g[cslot<M, P>(c, 0)], r[0]);
-  pr[0] = h[cslot<M, P>(c, 0)];
-  r[0] = y;
-#pragma unroll
-  for (int m = 1; m < M; ++m) {
-    const int k = cslot<M, P>(c, m);
-    const double2 hm = h[k];
-    y = cfma(hm, y, cmul(g[k], r[m]));
-    pr[m] = cmul(hm, pr[m - 1]);
-    r[m] = y;
-  }
-  Affine ex = exclusive_scan<P, false>(Affine{pr[M - 1], y}, scratch);
-  const double2 y_in = ex.b;
-#pragma unroll
-  for (int m = 0; m < M; ++m) r[m] = cfma(pr[m], y_in, r[m]);
-  // backward, zero carry-in: x_i = y_i + h_i x_{i+1}
-  double2 x = r[M - 1];
-  pr[M - 1] = h[cslot<M, P>(c, M - 1)];
-#pragma unroll
-  for (int m = M - 2; m >= 0; --m) {
-    const double2 hm = h[cslot<M, P>(c, m)];
-    x = cfma(hm, x, r[m]);
-    pr[m] = cmul(hm, pr[m + 1]);
-    r[m] = x;
-  }
-  ex = exclusive_scan<P, true>(Affine{pr[0], x}, scratch);
-  const double2 x_in = ex.b;
-#pragma unroll
-  for (int m = 0; m < M; ++m) r[m] = cfma(pr[m], x_in, r[m]);
 }
 
 }  // namespace pxp

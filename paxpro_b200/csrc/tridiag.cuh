@@ -1,9 +1,8 @@
-// tridiag.cuh -- parallel complex tridiagonal solve used by the CN and ADI
-// kernels (replacing the serial ThomasAlgorithm::solve sweep,
+// tridiag.cuh -- parallel complex tridiagonal solve of the step-by-step
+// Crank-Nicolson kernel (replacing the serial ThomasAlgorithm::solve sweep,
 // include/thomasAlgorithm.tpp:2-32).
 //
-// Systems have a symmetric, constant off-diagonal `sub` (CN: -i rho/4,
-// ADI: -i/(2 k d^2)) and per-row diagonals / right-hand sides.  A system of L
+// Systems have a symmetric, constant off-diagonal `sub` (-i rho/4) and per-row diagonals / right-hand sides.  A system of L
 // unknowns is split into P chunks of M consecutive rows, one chunk per
 // thread.  Each thread eliminates its chunk interior in registers (partition
 // method: interior x_i = y_i + p_i x_first + q_i x_last, three right-hand
