@@ -708,7 +708,8 @@ __device__ __forceinline__ void adi_group_solve(double2 (&r)[SCAP][M], const Adi
 // Systems per group S: a thread owns one chunk of M rows of the S systems of
 // its group; NG = ceil(G / S) groups of P = n/M threads each (the last group
 // may hold fewer systems).
-template <int N, int M, int G, int S, bool XH>
+// Complex64 fields are widened as they are staged and rounded as they leave.
+template <typename R, int N, int M, int G, int S, bool XH>
 __global__ void __launch_bounds__(((G + S - 1) / S) * (N / M), 1)
     adi_const_wave_kernel(const AdiHalf h, const double2 *__restrict__ tabs) {
   using L = AdiWaveTile<N, M, G, XH>;
@@ -729,8 +730,13 @@ __global__ void __launch_bounds__(((G + S - 1) / S) * (N / M), 1)
   const int tid = threadIdx.x;
   const int group = tid / P, gtid = tid % P;
   const int s_base = blockIdx.x * G;
-  const double2 *in = reinterpret_cast<const double2 *>(h.in);
-  double2 *out = reinterpret_cast<double2 *>(h.out);
+  using C = typename Cx<R>::T;
+  const C *in = reinterpret_cast<const C *>(h.in);
+  C *out = reinterpret_cast<C *>(h.out);
+  auto stage = [](double2 *dst, const C *src) {
+    if constexpr (sizeof(R) == 8) adi_cp_async16(dst, src);
+    else *dst = to_d(*src);
+  };
   const int nr = h.n;  // systems, and positions per system (N: rows solved)
   // staged systems s_base - 1 + g exist for g in [g_lo, g_hi)
   const int g_lo = s_base == 0 ? 1 : 0;
@@ -759,15 +765,15 @@ __global__ void __launch_bounds__(((G + S - 1) / S) * (N / M), 1)
     constexpr int PPI = T / RW;  // positions per pass
     const int g = tid % RW;
     if (tid < PPI * RW && g >= g_lo && g < g_hi) {
-      const double2 *src = in + (s_base - 1 + g);
+      const C *src = in + (s_base - 1 + g);
       for (int p = tid / RW; p < nr; p += PPI)
-        adi_cp_async16(tile + L::at(p / M, p % M, g), src + (long long)p * h.stride_pos);
+        stage(tile + L::at(p / M, p % M, g), src + (long long)p * h.stride_pos);
     }
   } else {
 #pragma unroll 1
     for (int g = g_lo; g < g_hi; ++g) {
-      const double2 *src = in + (long long)(s_base - 1 + g) * h.stride_sys;
-      for (int p = tid; p < nr; p += T) adi_cp_async16(tile + L::at(p / M, p % M, g), src + p);
+      const C *src = in + (long long)(s_base - 1 + g) * h.stride_sys;
+      for (int p = tid; p < nr; p += T) stage(tile + L::at(p / M, p % M, g), src + p);
     }
   }
   asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -800,7 +806,7 @@ __global__ void __launch_bounds__(((G + S - 1) / S) * (N / M), 1)
       for (int m = 0; m < M; ++m) tile[L::at(gtid, m, group * S + j + 1)] = r[j][m];
     }
   __syncthreads();
-  double2 *save = reinterpret_cast<double2 *>(h.save);
+  C *save = reinterpret_cast<C *>(h.save);
   const int nsys = nr - s_base < G ? nr - s_base : G;  // the last CTA may hold fewer
   if constexpr (XH) {
     // consecutive threads write consecutive systems of a position
@@ -808,7 +814,7 @@ __global__ void __launch_bounds__(((G + S - 1) / S) * (N / M), 1)
     const int gg = tid % G;
     if (tid < PPI * G && gg < nsys) {
       for (int p = tid / G; p < nr; p += PPI) {
-        const double2 v = tile[L::at(p / M, p % M, gg + 1)];
+        const C v = from_d<R>(tile[L::at(p / M, p % M, gg + 1)]);
         const long long off = (long long)p * h.stride_pos + s_base + gg;
         out[off] = v;
         if (save) save[off] = v;
@@ -819,7 +825,7 @@ __global__ void __launch_bounds__(((G + S - 1) / S) * (N / M), 1)
     for (int gg = 0; gg < nsys; ++gg) {
       const long long base = (long long)(s_base + gg) * h.stride_sys;
       for (int p = tid; p < nr; p += T) {
-        const double2 v = tile[L::at(p / M, p % M, gg + 1)];
+        const C v = from_d<R>(tile[L::at(p / M, p % M, gg + 1)]);
         out[base + p] = v;
         if (save) save[base + p] = v;
       }
@@ -1001,7 +1007,7 @@ static bool adi_pipe_enabled() {
   return on;
 }
 
-template <int N, int M, int G, int S, bool XH>
+template <typename R, int N, int M, int G, int S, bool XH>
 static cudaError_t adi_const_wave_launch_x(const AdiHalf &h, const void *tabs, cudaStream_t s) {
   constexpr int P = N / M, NG = (G + S - 1) / S, T = NG * P;
   constexpr size_t smem = adi_wave_bar_bytes<NG>() +
@@ -1010,10 +1016,16 @@ static cudaError_t adi_const_wave_launch_x(const AdiHalf &h, const void *tabs, c
   static_assert(smem + 16 <= 227 * 1024, "staged ADI tile exceeds shared memory");
   static_assert(P % 32 == 0, "whole warps per group");
   static_assert(NG <= 15, "one named barrier per group");
-  auto k = adi_pipe_enabled() ? adi_pipe_wave_kernel<N, M, G, S, XH>
-                              : adi_const_wave_kernel<N, M, G, S, XH>;
+  auto k = adi_const_wave_kernel<R, N, M, G, S, XH>;
+  if constexpr (sizeof(R) == 8)
+    if (adi_pipe_enabled()) k = adi_pipe_wave_kernel<N, M, G, S, XH>;
   {
-    const cudaError_t attr = raise_dynamic_smem((const void *)k, (int)smem);
+    cudaError_t attr = raise_dynamic_smem((const void *)k, (int)smem);
+    // room for one CTA an SM: in a larger carve-out, left behind by a kernel
+    // that wanted it (the general half step's), the next half step's CTAs start
+    // two to an SM beside this one's and leave other SMs idle (512 nodes after
+    // a plane with material: 10.7 -> 13.7 us a step)
+    if (attr == cudaSuccess) attr = prefer_smem_carveout((const void *)k, (int)smem, 1);
     if (attr != cudaSuccess) return attr;
   }
   // launched as a programmatic dependent of the previous kernel in the
@@ -1031,11 +1043,11 @@ static cudaError_t adi_const_wave_launch_x(const AdiHalf &h, const void *tabs, c
   return cudaLaunchKernelEx(&cfg, k, h, (const double2 *)tabs);
 }
 
-template <int N, int M, int G, int S>
+template <typename R, int N, int M, int G, int S>
 static cudaError_t adi_const_wave_launch(const AdiHalf &h, const void *tabs, cudaStream_t s) {
   if (tabs == nullptr) return cudaErrorInvalidValue;
-  return h.stride_sys == 1 ? adi_const_wave_launch_x<N, M, G, S, true>(h, tabs, s)
-                           : adi_const_wave_launch_x<N, M, G, S, false>(h, tabs, s);
+  return h.stride_sys == 1 ? adi_const_wave_launch_x<R, N, M, G, S, true>(h, tabs, s)
+                           : adi_const_wave_launch_x<R, N, M, G, S, false>(h, tabs, s);
 }
 
 // (M, G) of the one-wave kernel per size: each system group holds whole
@@ -1136,41 +1148,37 @@ cudaError_t launch_wait_selftest(unsigned long long limit_ns, unsigned *timeouts
   return cudaGetLastError();
 }
 
+template <typename R>
+static cudaError_t adi_half_const(const AdiHalf &h, const void *g, const void *hh,
+                                  const void *staged, cudaStream_t s) {
+  switch (adi_wave_n(h.n)) {
+    case 64: return adi_const_wave_launch<R, 64, 2, 4, 2>(h, staged, s);
+    case 128: return adi_const_wave_launch<R, 128, 4, 2, 1>(h, staged, s);
+    case 256: return adi_const_wave_launch<R, 256, 8, 2, 1>(h, staged, s);
+    // systems a CTA: as few as still make one wave of the 148 SMs (us a step:
+    // 290 nodes 9.7 with four, 7.2 with two; 513 16.0 with six, 12.9 with
+    // four; 800 23.0 with seven, 19.2 with six); three at 297 .. 444 nodes,
+    // a full group of two and a half empty one, are slower than four (440:
+    // 12.1 against 11.2)
+    case 512:
+      if (h.n <= 296) return adi_const_wave_launch<R, 512, 8, 2, 1>(h, staged, s);
+      return adi_const_wave_launch<R, 512, 8, 4, 2>(h, staged, s);
+    case 768:
+      if (h.n <= 592) return adi_const_wave_launch<R, 768, 8, 4, 2>(h, staged, s);
+      if (h.n <= 740) return adi_const_wave_launch<R, 768, 8, 5, 2>(h, staged, s);
+      return adi_const_wave_launch<R, 768, 8, 6, 2>(h, staged, s);
+    case 1024:
+      if (h.n <= 888) return adi_const_wave_launch<R, 1024, 8, 6, 2>(h, staged, s);
+      return adi_const_wave_launch<R, 1024, 8, 7, 2>(h, staged, s);
+    default: break;
+  }
+  return h.n == 2048 ? adi_const_launch<R, 2048, 2>(h, g, hh, s) : cudaErrorInvalidValue;
+}
+
 cudaError_t launch_adi_half_const(Precision p, const AdiHalf &h, const void *g, const void *hh,
                                   const void *staged, cudaStream_t s) {
-#define PXP_AC(NN, GG)                                                                  \
-  case NN:                                                                              \
-    return p == kFP64 ? adi_const_launch<double, NN, GG>(h, g, hh, s)                   \
-                      : adi_const_launch<float, NN, GG>(h, g, hh, s);
-  if (p == kFP64) {
-    switch (adi_wave_n(h.n)) {
-      case 64: return adi_const_wave_launch<64, 2, 4, 2>(h, staged, s);
-      case 128: return adi_const_wave_launch<128, 4, 2, 1>(h, staged, s);
-      case 256: return adi_const_wave_launch<256, 8, 2, 1>(h, staged, s);
-      // systems a CTA: as few as still make one wave of the 148 SMs (us a step:
-      // 290 nodes 9.7 with four, 7.2 with two; 513 16.0 with six, 12.9 with
-      // four; 800 23.0 with seven, 19.2 with six); three at 297 .. 444 nodes,
-      // a full group of two and a half empty one, are slower than four (440:
-      // 12.1 against 11.2)
-      case 512:
-        if (h.n <= 296) return adi_const_wave_launch<512, 8, 2, 1>(h, staged, s);
-        return adi_const_wave_launch<512, 8, 4, 2>(h, staged, s);
-      case 768:
-        if (h.n <= 592) return adi_const_wave_launch<768, 8, 4, 2>(h, staged, s);
-        if (h.n <= 740) return adi_const_wave_launch<768, 8, 5, 2>(h, staged, s);
-        return adi_const_wave_launch<768, 8, 6, 2>(h, staged, s);
-      case 1024:
-        if (h.n <= 888) return adi_const_wave_launch<1024, 8, 6, 2>(h, staged, s);
-        return adi_const_wave_launch<1024, 8, 7, 2>(h, staged, s);
-      default: break;
-    }
-  }
-  switch (h.n) {
-    PXP_AC(64, 4) PXP_AC(128, 4) PXP_AC(256, 4) PXP_AC(512, 4) PXP_AC(1024, 4) PXP_AC(2048, 2)
-    default:
-      return cudaErrorInvalidValue;
-  }
-#undef PXP_AC
+  return p == kFP64 ? adi_half_const<double>(h, g, hh, staged, s)
+                    : adi_half_const<float>(h, g, hh, staged, s);
 }
 
 template <typename R, int M, int W, int G>
@@ -1198,7 +1206,7 @@ static cudaError_t adi_chunk_launch_t(const AdiHalf &h, cudaStream_t s) {
 
 bool adi_size_supported(int n) { return n >= 4 && n <= 2048; }
 
-bool adi_supported(Precision, int n) { return n >= 64 && n <= 2048 && !(n & (n - 1)); }
+bool adi_const_supported(int n) { return adi_wave_n(n) > 0 || n == 2048; }
 
 // Rows a thread, warps a system and systems a CTA per grid size.  Two CTAs an
 // SM beat one larger CTA (513: G = 2 21.1 us a step, G = 4 22.8) except where

@@ -1461,10 +1461,7 @@ int pxp_solver_create(const pxp_problem *problem, pxp_solver *out) {
       if ((rc = alloc(h, &h->d_field2, h->csize * h->npts, "second field buffer")))
         return cleanup_fail(rc);
       // vacuum factor tables for the step-invariant kernels (grids those run)
-      // the vacuum fast path: powers of two in both precisions, any size the
-      // FP64 one-wave kernel takes
-      if (pxp::adi_supported(h->prec, (int)h->nx) ||
-          (h->prec == pxp::kFP64 && pxp::adi_wave_n((int)h->nx) > 0))
+      if (pxp::adi_const_supported((int)h->nx))
         if ((rc = adi_build_lu(h))) return cleanup_fail(rc);
       break;
     case PXP_FFT_SOLVER_3D:

@@ -202,18 +202,16 @@ struct AdiHalf {
   Sphere spheres[kInlineSpheres];
 };
 cudaError_t launch_adi_half(Precision p, const AdiHalf &h, cudaStream_t s);
-// Grid sizes the general kernel takes (any n from 4 to 2048) and the powers
-// of two among them that the FP32 vacuum kernel takes.
+// Grid sizes the general kernel takes (any n from 4 to 2048) and those of the
+// vacuum kernels (up to 1024, and 2048).
 bool adi_size_supported(int n);
-bool adi_supported(Precision p, int n);
+bool adi_const_supported(int n);
 // Half step whose plane holds no material and no transparent boundary: the
 // matrix is the same for every system and every step; g/h are its Thomas
-// factor tables (n complex128 each, see scan_solve.cuh; read by the FP32
-// kernel, which takes powers of two only).
-// `staged`: the factor tables of the FP64 one-wave kernel, for its padded
-// system length adi_wave_n(n), with their in-chunk products, in the layout
-// it copies into shared memory (adi_const_staged_tables).  FP64 runs any
-// n with adi_wave_n(n) > 0 here.
+// factor tables (n complex128 each, see scan_solve.cuh; read at 2048 nodes).
+// `staged`: the factor tables of the one-wave kernel, for its padded system
+// length adi_wave_n(n), with their in-chunk products, in the layout it copies
+// into shared memory (adi_const_staged_tables).
 cudaError_t launch_adi_half_const(Precision p, const AdiHalf &h, const void *g, const void *hh,
                                   const void *staged, cudaStream_t s);
 // System length of the FP64 one-wave vacuum kernel for a grid of n nodes

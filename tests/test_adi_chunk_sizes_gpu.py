@@ -32,12 +32,19 @@ def test_general_half_step_at_launch_shape_edges(n, use_tbc, precision):
             assert _int_rel(a, b) <= FP32_INT_TOL
 
 
-@pytest.mark.parametrize("n", [257, 296, 297, 513, 592, 593, 740, 741, 769, 888, 889])
-def test_vacuum_half_step_at_launch_shape_edges(n):
-    """The one-wave vacuum kernel where its systems a CTA change."""
+@pytest.mark.parametrize("n,precision", [(n, 0) for n in (257, 296, 297, 513, 592, 593, 740, 741, 769,
+                                                          888, 889)] +
+                         [(n, 1) for n in (5, 64, 100, 256, 296, 513, 741, 888, 1024, 2048)])
+def test_vacuum_half_step_at_launch_shape_edges(n, precision):
+    """The one-wave vacuum kernel where its systems a CTA change, and on
+    complex64 fields (2048 nodes: the kernel above its sizes)."""
     x = -500.0 + wl.step_for_nodes(-500.0, 500.0, n) * np.arange(n)
     g = np.exp(-((x - 40.0) / 300.0) ** 2) * np.exp(1j * 2e-3 * x)
     u0 = np.asfortranarray(g[:, None] * g[None, :])
-    out, saves, ref_out, ref_saves = _run_both(n, 0.0, 4, 1000.0, [], u0=u0)
+    out, saves, ref_out, ref_saves = _run_both(n, 0.0, 4, 1000.0, [], u0=u0, precision=precision)
     assert len(saves) == len(ref_saves) == 4
-    assert max(_rel(a, b) for a, b in zip(saves, ref_saves)) <= FP64_TOL
+    for a, b in zip(saves, ref_saves):
+        if precision == 0:
+            assert _rel(a, b) <= FP64_TOL
+        else:
+            assert _int_rel(a, b) <= FP32_INT_TOL
