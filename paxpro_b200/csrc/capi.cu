@@ -696,7 +696,7 @@ int adi_build_lu(pxp_solver_s *h) {
   thomas_factor(dgx, -0.5 * im / (k * dx * dx), gx);
   thomas_factor(dgy, -0.5 * im / (k * dy * dy), gy);
   // [gx | hx | gy | hy] in natural order, then the x and y tables staged for
-  // the FP64 one-wave kernel ([g | h | pf | pb] each, for its system length
+  // the one-wave kernel ([g | h | pf | pb] each, for its system length
   // nw; rows n .. nw-1 decoupled: g = 1, h = 0)
   const unsigned nw = (unsigned)adi_tab_len(n);
   std::vector<cd> tabs(4 * (size_t)n + 8 * (size_t)nw);

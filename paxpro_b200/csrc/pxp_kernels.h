@@ -214,7 +214,7 @@ bool adi_const_supported(int n);
 // into shared memory (adi_const_staged_tables).
 cudaError_t launch_adi_half_const(Precision p, const AdiHalf &h, const void *g, const void *hh,
                                   const void *staged, cudaStream_t s);
-// System length of the FP64 one-wave vacuum kernel for a grid of n nodes
+// System length of the one-wave vacuum kernel for a grid of n nodes
 // (64, 128, 256, 512, 768 or 1024, the smallest that holds n), 0 when n is
 // outside 4 .. 1024.  Rows n .. length-1 are decoupled padding.
 int adi_wave_n(int n);
