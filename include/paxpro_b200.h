@@ -105,7 +105,10 @@ int pxp_solver_destroy(pxp_solver s);
 /* Material hook, z-invariant medium sampled per transverse point
  * (ParaxialSimulation::getXrayMatProp, src/paraxialSimulation.cpp:513-537):
  * delta[i], beta[i] at x_i for the 2-D kinds (n = Nx), or at (x_col, y_row)
- * column-major for the 3-D kinds (n = Nx*Ny). */
+ * column-major for the 3-D kinds (n = Nx*Ny).
+ * A material call (any of the four) that fails after it has begun to replace
+ * the medium (device memory) leaves none: steps then fail with PXP_ERR_INVALID
+ * until a material call succeeds. */
 int pxp_set_material_table(pxp_solver s, const double *delta, const double *beta, size_t n);
 
 /* Material hook, sampled per step for z-varying media (any MaterialFunction

@@ -80,7 +80,7 @@ struct pxp_solver_s {
   bool cn_const = false;                     // CN matrix step-invariant
   bool cn_two_planes = false;                // its one step's two planes differ
   bool cn_vacuum = false;                    // no material set yet: its tables are built
-                                             // when it steps without one
+                                             // when it steps without one (cn_const holds)
   size_t dev_bytes = 0;                      // device memory held by the handle
   pxp::Fft1dJob job_fft{};                   // host copies of the job descriptors
   pxp::CnJob job_cn{};
@@ -108,6 +108,9 @@ struct pxp_solver_s {
   int planes3_per = 0;
   bool planes3_invariant = false;  // one plane (a z-invariant table) for every step
   bool material_set = false;
+  // false from the moment a material call starts to replace the medium until it
+  // has done so: after a failed one the old tables and planes are gone
+  bool medium_ok = true;
   bool ic_set = false;
   unsigned current_step = 1;
   // the device's count of ran-out kernel waits (wait_counter.cu): the host's
@@ -537,6 +540,7 @@ int fft1d_set_trans(pxp_solver_s *h, const double *delta, const double *beta, in
       if (h->prec == pxp::kFP32) v = v / (double)n;
       t[j] = v;
     }
+  h->medium_ok = false;
   free_dev(h->d_trans, h->stream);
   int rc;
   if ((rc = alloc(h, &h->d_trans, table_entry_bytes(h) * t.size(), "transmission table")))
@@ -573,8 +577,10 @@ int fft1d_write_job(pxp_solver_s *h) {
 // ---- CN --------------------------------------------------------------------
 int cn_build_lu(pxp_solver_s *h, const double *delta, const double *beta);
 
+// vacuum: the medium of a handle that no material was set on; its factor
+// tables wait for a step without one (cn_vacuum_tables).
 int cn_set_planes(pxp_solver_s *h, const double *delta, const double *beta, int nsteps,
-                  int first_step, bool two_planes_per_step) {
+                  int first_step, bool two_planes_per_step, bool vacuum = false) {
   // Device layout: 4 blocks [delta | beta | delta_prev | beta_prev], each
   // nsteps * n doubles; per-step stride n.
   const unsigned n = h->nx;
@@ -588,6 +594,8 @@ int cn_set_planes(pxp_solver_s *h, const double *delta, const double *beta, int 
     std::memcpy(&buf[2 * per + (size_t)s * n], delta + src1, sizeof(double) * n);
     std::memcpy(&buf[3 * per + (size_t)s * n], beta + src1, sizeof(double) * n);
   }
+  h->medium_ok = false;
+  h->cn_const = h->cn_vacuum = false;
   free_dev(h->d_mat, h->stream);
   int rc;
   if ((rc = alloc(h, (void **)&h->d_mat, sizeof(double) * buf.size(), "material planes")))
@@ -598,12 +606,12 @@ int cn_set_planes(pxp_solver_s *h, const double *delta, const double *beta, int 
   h->mat_step0 = first_step;
   h->material_set = true;
   // step-invariant matrix when the same plane serves every step
-  h->cn_const = false;
   h->cn_two_planes = std::memcmp(&buf[0], &buf[2 * per], sizeof(double) * 2 * per) != 0;
   if (nsteps == 1 && pxp::cn_const_supported(h->prec, pxp::cn_padded_n((int)n))) {
-    if (!h->cn_vacuum)
+    if (!vacuum)
       if (int rc2 = cn_build_lu(h, delta, beta)) return rc2;
     h->cn_const = true;
+    h->cn_vacuum = vacuum;
   }
   return PXP_OK;
 }
@@ -1453,8 +1461,7 @@ int pxp_solver_create(const pxp_problem *problem, pxp_solver *out) {
       break;
     case PXP_CRANK_NICHOLSON:
       if ((rc = alloc(h, &h->d_job, sizeof(pxp::CnJob), "job descriptor"))) return cleanup_fail(rc);
-      h->cn_vacuum = true;
-      if ((rc = cn_set_planes(h, zeros.data(), zeros.data(), 1, 1, false))) return cleanup_fail(rc);
+      if ((rc = cn_set_planes(h, zeros.data(), zeros.data(), 1, 1, false, true))) return cleanup_fail(rc);
       if ((rc = cn_write_job(h))) return cleanup_fail(rc);
       break;
     case PXP_ADI:
@@ -1477,6 +1484,7 @@ int pxp_solver_create(const pxp_problem *problem, pxp_solver *out) {
       }
       break;
   }
+  h->medium_ok = true;
   *out = h;
   return PXP_OK;
 }
@@ -1516,10 +1524,24 @@ static int rewrite_job(pxp_solver_s *h) {
   }
 }
 
+// The end of a material call whose new tables and planes are in place.
+static int medium_replaced(pxp_solver_s *h) {
+  const int rc = rewrite_job(h);
+  h->medium_ok = rc == PXP_OK;
+  return rc;
+}
+
+// A handle whose last material call failed has no medium to step through.
+static int check_medium(pxp_solver_s *h) {
+  if (h->medium_ok) return PXP_OK;
+  return h->fail(PXP_ERR_INVALID, "the last material call failed: the medium must be set again");
+}
+
 // Copy nplanes sampled planes of a 3-D kind to the device ([delta planes |
 // beta planes]); the planes replace a sphere or CSG material.
 static int store_planes3(pxp_solver_s *h, const double *delta, const double *beta, size_t nplanes) {
   const size_t need = 2 * nplanes * (size_t)h->npts;
+  h->medium_ok = false;
   if (need > h->planes3_cap) {
     free_dev(h->d_planes3, h->stream);
     h->dev_bytes -= sizeof(double) * h->planes3_cap;
@@ -1556,7 +1578,6 @@ int pxp_set_material_table(pxp_solver h, const double *delta, const double *beta
       if ((rc = fft1d_set_trans(h, delta, beta, 1, 1))) return rc;
       break;
     case PXP_CRANK_NICHOLSON:
-      h->cn_vacuum = false;
       if ((rc = cn_set_planes(h, delta, beta, 1, 1, false))) return rc;
       break;
     case PXP_FFT_SOLVER_3D:
@@ -1567,14 +1588,14 @@ int pxp_set_material_table(pxp_solver h, const double *delta, const double *beta
       h->planes3_invariant = true;
       h->planes3_per = 1;
       h->plane_count = 0;
-      return PXP_OK;
+      return medium_replaced(h);
     default:
       return h->fail(PXP_ERR_UNSUPPORTED, "material tables not supported for this kind");
   }
   h->h_delta.assign(delta, delta + n);
   h->h_beta.assign(beta, beta + n);
   h->plane_count = 0;
-  return rewrite_job(h);
+  return medium_replaced(h);
 }
 
 int pxp_set_material_planes(pxp_solver h, const double *delta, const double *beta,
@@ -1589,7 +1610,6 @@ int pxp_set_material_planes(pxp_solver h, const double *delta, const double *bet
       if (nsteps == 1) h->trans_stride = 0;
       break;
     case PXP_CRANK_NICHOLSON:
-      h->cn_vacuum = false;
       if ((rc = cn_set_planes(h, delta, beta, nsteps, first_step, true))) return rc;
       break;
     case PXP_FFT_SOLVER_3D:
@@ -1600,14 +1620,14 @@ int pxp_set_material_planes(pxp_solver h, const double *delta, const double *bet
       h->planes3_invariant = false;
       h->plane_first = first_step;
       h->plane_count = nsteps;
-      return PXP_OK;
+      return medium_replaced(h);
     }
     default:
       return h->fail(PXP_ERR_UNSUPPORTED, "material planes not supported for this kind");
   }
   h->plane_first = first_step;
   h->plane_count = nsteps;
-  return rewrite_job(h);
+  return medium_replaced(h);
 }
 
 int pxp_set_material_spheres(pxp_solver h, const pxp_sphere *spheres, int n) {
@@ -1615,6 +1635,7 @@ int pxp_set_material_spheres(pxp_solver h, const pxp_sphere *spheres, int n) {
   if (h->prob.kind != PXP_ADI && h->prob.kind != PXP_FFT_SOLVER_3D)
     return h->fail(PXP_ERR_UNSUPPORTED, "sphere materials apply to the 3-D kinds");
   PXP_TRY_CUDA(h, cudaStreamSynchronize(h->stream));
+  h->medium_ok = false;
   h->plane_count = 0;  // a sphere list replaces sampled planes
   h->planes3_invariant = false;
   h->spheres.assign(spheres, spheres + n);
@@ -1633,7 +1654,7 @@ int pxp_set_material_spheres(pxp_solver h, const pxp_sphere *spheres, int n) {
     if (int rc_ = h2d(h, h->d_spheres, dev.data(), sizeof(pxp::Sphere) * n)) return rc_;
   }
   h->material_set = true;
-  return PXP_OK;
+  return medium_replaced(h);
 }
 
 namespace {
@@ -1698,6 +1719,7 @@ int pxp_set_material_csg(pxp_solver h, const pxp_csg_module *modules, int nmodul
         (shapes[k].operation != PXP_CSG_UNION && shapes[k].operation != PXP_CSG_DIFFERENCE))
       return h->fail(PXP_ERR_INVALID, "CSG shape " + std::to_string(k) + ": bad kind or operation");
   PXP_TRY_CUDA(h, cudaStreamSynchronize(h->stream));
+  h->medium_ok = false;
   h->plane_count = 0;  // a CSG material replaces sampled planes
   h->planes3_invariant = false;
   // z range per module: the union of its parts' union shapes' ranges (a
@@ -1747,7 +1769,7 @@ int pxp_set_material_csg(pxp_solver h, const pxp_csg_module *modules, int nmodul
   h->spheres.clear();
   free_dev(h->d_spheres, h->stream);
   h->material_set = true;
-  return PXP_OK;
+  return medium_replaced(h);
 }
 
 static int upload_field(pxp_solver_s *h, void *dst, const double *src) {
@@ -1811,6 +1833,7 @@ int pxp_step(pxp_solver h, int nsteps) {
   if (!h->ic_set)
     return h->fail(PXP_ERR_INVALID, "setInitialConditions must be called before stepping");
   if (nsteps == 0) return PXP_OK;
+  if (int rc = check_medium(h)) return rc;
   PXP_TRY_CUDA(h, cudaSetDevice(h->prob.device));
   const long long first = h->current_step, last = first + nsteps - 1;
   if (h->plane_count > 0 &&
@@ -2497,6 +2520,7 @@ int pxp_batch_admit(pxp_batch b, pxp_solver h, int nsteps) {
   if (b == nullptr || h == nullptr || nsteps < 0) return PXP_ERR_INVALID;
   if (h->prob.device != b->device) return b->fail(PXP_ERR_INVALID, "solver on another device");
   if (!h->ic_set) return b->fail(PXP_ERR_INVALID, "solver has no initial conditions");
+  if (int rc = check_medium(h)) return b->fail(rc, h->err);
   for (pxp_solver_s *a : b->active)
     if (a == h) return b->fail(PXP_ERR_INVALID, "solver already admitted");
   if (h->plane_count > 0 &&
@@ -2522,6 +2546,9 @@ int pxp_batch_admit(pxp_batch b, pxp_solver h, int nsteps) {
 int pxp_batch_round(pxp_batch b, int max_steps) {
   if (b == nullptr || max_steps <= 0) return PXP_ERR_INVALID;
   cudaSetDevice(b->device);
+  for (pxp_solver_s *h : b->active)
+    if (h->batch_remaining > 0)
+      if (int rc = check_medium(h)) return b->fail(rc, h->err);
   // the staging buffer of the previous round must be consumed
   if (cudaStreamSynchronize(b->stream) != cudaSuccess) return b->fail(PXP_ERR_CUDA, "batch stream");
   // ---- 2-D groups: key (kind, n, precision, CN matrix path)
