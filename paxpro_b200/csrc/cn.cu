@@ -370,32 +370,32 @@ __device__ __forceinline__ double cn_finish(const CnJob &job, int step, double2 
   return acc;
 }
 
-// The flux sum of a step over the K CTAs of a cluster (part: K slots in CTA
-// 0's shared memory).
-template <int T, int K>
-__device__ __forceinline__ void cn_flux(const CnJob &job, int step, double acc, double (*red)[flux_slots<T>()],
-                                        double *part, int rank) {
-  double *row = red[step & 1];
-  flux_warp_total<T>(acc, row);
-  __syncthreads();
+// The flux sum of a step: every warp's total goes to its slot in CTA 0's shared
+// memory (part: rows of alternating steps) and one tree adds the slots, so the
+// sum does not depend on how many CTAs the problem's warps are spread over.  A
+// row is written again only after a later step's scan, whose barrier follows
+// its reads.
+template <int TW, int K>
+__device__ __forceinline__ void cn_flux(const CnJob &job, int step, double acc, double (*part)[TW],
+                                        int gw) {
+  double *row = part[step & 1];
+  const int lane = threadIdx.x & 31;
+  double v = acc;
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
   if constexpr (K == 1) {
-    flux_store<T>(job.flux, step, row);
+    if (lane == 0) row[gw] = v;
+    __syncthreads();
   } else {
     cg::cluster_group cluster = cg::this_cluster();
-    if (threadIdx.x < 32) {
-      double v = threadIdx.x < flux_slots<T>() ? row[threadIdx.x] : 0.0;
-#pragma unroll
-      for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
-      if (threadIdx.x == 0) *cluster.map_shared_rank(part + rank, 0) = v;
-    }
-    cluster.sync();  // every CTA's total is in CTA 0's slots
-    if (rank == 0 && threadIdx.x == 0) {
-      double v = 0.0;
-      for (int j = 0; j < K; ++j) v += part[j];
-      job.flux.out[step - job.flux.step0] = v;
-    }
-    cluster.sync();  // and read, before the next step's
+    if (lane == 0) *cluster.map_shared_rank(row + gw, 0) = v;
+    cluster.sync();
   }
+  if (gw != 0) return;  // the first warp of CTA 0
+  v = lane < TW ? row[lane] : 0.0;
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
+  if (lane == 0) job.flux.out[step - job.flux.step0] = v;
 }
 
 // z-invariant medium: tables and scan products set up once, the field in
@@ -419,8 +419,7 @@ __global__ void __launch_bounds__(T) cn_const_kernel(const CnJob *__restrict__ j
   double2 *sR = sL + NC;
   double2 *sW = sR + NC;
   double2 *tot = sW + NC;  // 2 x 2 x TW
-  __shared__ double flux_red[2][flux_slots<T>()];
-  __shared__ double flux_part[K];
+  __shared__ double flux_part[2][TW];
   CnJob job = jobs[blockIdx.x / K];
   if (nsteps_ov >= 0) {
     job.step0 = step0_ov;
@@ -487,7 +486,7 @@ __global__ void __launch_bounds__(T) cn_const_kernel(const CnJob *__restrict__ j
         tot + par * 2 * TW, gw, publish, sync, [] {});
     const double acc = cn_finish<R>(job, step, u, x, s0, nreal, flux, fw);
     if constexpr (FLUX)
-      if (flux) cn_flux<T, K>(job, step, acc, flux_red, flux_part, rank);
+      if (flux) cn_flux<TW, K>(job, step, acc, flux_part, gw);
   }
   if constexpr (K > 1) cg::this_cluster().sync();  // no CTA leaves while a peer writes to it
 #pragma unroll
@@ -676,8 +675,7 @@ __global__ void __launch_bounds__(T) cn_planes_kernel(const CnJob *__restrict__ 
   double2 *sW = sC + NC;
   double2 *sP = sW + NC;            // 14 x T
   double2 *tot = sP + kCnCoefs * T;  // 2 x 2 x TW
-  __shared__ double flux_red[2][flux_slots<T>()];
-  __shared__ double flux_part[K];
+  __shared__ double flux_part[2][TW];
   const CnJob job = jobs[0];
   const int t = threadIdx.x, rank = K > 1 ? (int)(blockIdx.x % K) : 0;
   const int gw = rank * W + t / 32, tt = rank * T + t;
@@ -757,7 +755,7 @@ __global__ void __launch_bounds__(T) cn_planes_kernel(const CnJob *__restrict__ 
     fetch_w(st + 1);
     const double acc = cn_finish<R>(job, step, u, x, s0, nreal, flux, fw);
     if constexpr (FLUX)
-      if (flux) cn_flux<T, K>(job, step, acc, flux_red, flux_part, rank);
+      if (flux) cn_flux<TW, K>(job, step, acc, flux_part, gw);
   }
   cn_cp_wait<0>();
   if constexpr (K > 1) cg::this_cluster().sync();  // no CTA leaves while a peer writes to it
