@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <map>
 #include <tuple>
@@ -111,6 +112,7 @@ struct pxp_solver_s {
   // false from the moment a material call starts to replace the medium until it
   // has done so: after a failed one the old tables and planes are gone
   bool medium_ok = true;
+  bool counted = false;  // among handle_count
   bool ic_set = false;
   unsigned current_step = 1;
   // the device's count of ran-out kernel waits (wait_counter.cu): the host's
@@ -1150,6 +1152,23 @@ int fft3d_variant(pxp_solver_s *h, const pxp::Fft3dPass &q0, const void *kx2, co
 
 bool cn_uses_const(const pxp_solver_s *h);
 
+// Handles of the process per device and dimension.  They may be stepping on
+// streams of their own beside a launch, which takes its size from them
+// (launch_cn_const); results never depend on it.
+constexpr int kMaxDevices = 64;  // as wait_counter
+std::atomic<int> g_handles_2d[kMaxDevices], g_handles_3d[kMaxDevices];
+
+std::atomic<int> &handle_count(const pxp_solver_s *h) {
+  const bool d2 = h->prob.kind == PXP_FFT_SOLVER_2D || h->prob.kind == PXP_CRANK_NICHOLSON;
+  return (d2 ? g_handles_2d : g_handles_3d)[h->prob.device];
+}
+
+// SMs that the device's handles other than the nj of a launch may be using.
+int sms_of_others(int device, int nj) {
+  constexpr int kAll = 1 << 20;
+  return g_handles_3d[device] > 0 ? kAll : std::max(0, g_handles_2d[device] - nj);
+}
+
 int cn_write_job(pxp_solver_s *h);
 
 // A CrankNicholson solver that steps before any material is set: its vacuum
@@ -1485,12 +1504,15 @@ int pxp_solver_create(const pxp_problem *problem, pxp_solver *out) {
       break;
   }
   h->medium_ok = true;
+  ++handle_count(h);
+  h->counted = true;
   *out = h;
   return PXP_OK;
 }
 
 int pxp_solver_destroy(pxp_solver h) {
   if (h == nullptr) return PXP_OK;
+  if (h->counted) --handle_count(h);
   if (h->stream) cudaStreamSynchronize(h->stream);
   if (h->graph) cudaGraphExecDestroy(h->graph);
   h->graph = nullptr;
@@ -1856,7 +1878,7 @@ int pxp_step(pxp_solver h, int nsteps) {
       if (cn_uses_const(h)) {
         e = pxp::launch_cn_const(h->prec, (const pxp::CnJob *)h->d_job, 1,
                                  pxp::cn_padded_n((int)h->nx), (int)first, nsteps, h->stream,
-                                 h->flux_count > 0);
+                                 h->flux_count > 0, sms_of_others(h->prob.device, 1));
         break;
       }
       e = cudaErrorMemoryAllocation;
@@ -2655,7 +2677,8 @@ int pxp_batch_round(pxp_batch b, int max_steps) {
     }
     else if (k.cpath)
       e = pxp::launch_cn_const((pxp::Precision)k.prec, (const pxp::CnJob *)jobs, (int)list.size(),
-                               pxp::cn_padded_n(k.n), -1, -1, gst, any_flux);
+                               pxp::cn_padded_n(k.n), -1, -1, gst, any_flux,
+                               sms_of_others(b->device, (int)list.size()));
     else
       e = pxp::launch_cn((pxp::Precision)k.prec, (const pxp::CnJob *)jobs, (int)list.size(),
                          pxp::cn_padded_n(k.n), -1, -1, gst, any_flux);

@@ -28,6 +28,7 @@
 #include "flux.cuh"
 #include "pxp_kernels.h"
 #include <algorithm>
+#include <cstdlib>
 #include <cooperative_groups.h>
 
 #include "tridiag.cuh"
@@ -801,16 +802,25 @@ bool cn_const_supported(Precision, int n) {
 }
 
 // Rows a thread, threads a CTA and CTAs a problem.  From 4096 rows on a
-// problem alone is faster on more SMs (4096: 2.17 us a step on one, 1.72 on
+// problem alone is faster on more SMs (4096: 3.0 us a step on one, 1.72 on
 // two, 1.42 on four; 8192 in FP32: 2.93 on two, 2.09 on four; 16384: 2.79 on
-// four, 2.07 on eight), at more SM time a problem: the wide form runs while
-// every problem of the launch finds its SMs free (kSms of them).  Both forms
-// have the same chunks and warps and give the same bits.  2048 rows gain too
-// little (1.40 on one SM, 1.31 on two).
+// four, 2.07 on eight), at more SM time a problem.  The widest form runs for
+// which every problem of the launch finds its SMs free beside the `others` that
+// the caller's other handles may be using: an SM for each handle of a 2-D kind,
+// all of them for one of a 3-D kind.  (A 1024^2 ADI half step is one wave of 147
+// CTAs, an SM each: beside a problem on four SMs it takes two waves, 40 us a
+// step against 22.9.)  The forms have the same chunks and warps and give the
+// same bits.  2048 rows gain too little (1.40 on one SM, 1.31 on two).
 constexpr int kSms = 148;
 cudaError_t launch_cn_const(Precision p, const CnJob *d_jobs, int nj, int n, int step0, int nsteps,
-                            cudaStream_t s, bool flux) {
+                            cudaStream_t s, bool flux, int others) {
   if (nj <= 0) return cudaSuccess;
+  // PXP_CN_CLUSTER=0|1 pins the narrowest or the widest form
+  const char *pin = std::getenv("PXP_CN_CLUSTER");
+  auto wide = [&](int ctas) {
+    if (pin && (pin[0] == '0' || pin[0] == '1')) return pin[0] == '1';
+    return (long long)nj * ctas + others <= kSms;
+  };
 #define PXP_CT(MM, TT, KK)                                                                \
   p == kFP64 ? cn_const_launch_t<double, MM, TT, KK>(d_jobs, nj, step0, nsteps, s, flux) \
              : cn_const_launch_t<float, MM, TT, KK>(d_jobs, nj, step0, nsteps, s, flux)
@@ -821,9 +831,9 @@ cudaError_t launch_cn_const(Precision p, const CnJob *d_jobs, int nj, int n, int
     case 512: return PXP_CT(8, 64, 1);
     case 1024: return PXP_CT(8, 128, 1);
     case 2048: return PXP_CT(16, 128, 1);
-    case 4096: return nj * 4 <= kSms ? PXP_CT(8, 128, 4) : PXP_CT(8, 256, 2);
-    case 8192: return nj * 4 <= kSms ? PXP_CT(16, 128, 4) : PXP_CT(16, 256, 2);
-    case 16384: return nj * 8 <= kSms ? PXP_CT(16, 128, 8) : PXP_CT(16, 256, 4);
+    case 4096: return wide(4) ? PXP_CT(8, 128, 4) : wide(2) ? PXP_CT(8, 256, 2) : PXP_CT(8, 512, 1);
+    case 8192: return wide(4) ? PXP_CT(16, 128, 4) : PXP_CT(16, 256, 2);
+    case 16384: return wide(8) ? PXP_CT(16, 128, 8) : PXP_CT(16, 256, 4);
     default: return cudaErrorInvalidValue;
   }
 #undef PXP_CT
