@@ -82,6 +82,10 @@ struct pxp_solver_s {
   bool cn_two_planes = false;                // its one step's two planes differ
   bool cn_vacuum = false;                    // no material set yet: its tables are built
                                              // when it steps without one (cn_const holds)
+  // sampled CN media: tables of the steps cn_win_first .. + cn_win_count - 1 in
+  // a buffer for cn_win_cap steps, the workspace of their factoring behind them
+  double2 *d_win = nullptr;
+  int cn_win_cap = 0, cn_win_first = 0, cn_win_count = 0;
   size_t dev_bytes = 0;                      // device memory held by the handle
   pxp::Fft1dJob job_fft{};                   // host copies of the job descriptors
   pxp::CnJob job_cn{};
@@ -579,6 +583,11 @@ int fft1d_write_job(pxp_solver_s *h) {
 // ---- CN --------------------------------------------------------------------
 int cn_build_lu(pxp_solver_s *h, const double *delta, const double *beta);
 
+void cn_win_release(pxp_solver_s *h, cudaStream_t s) {
+  free_dev(h->d_win, s);
+  h->cn_win_cap = h->cn_win_count = 0;
+}
+
 // vacuum: the medium of a handle that no material was set on; its factor
 // tables wait for a step without one (cn_vacuum_tables).
 int cn_set_planes(pxp_solver_s *h, const double *delta, const double *beta, int nsteps,
@@ -598,6 +607,7 @@ int cn_set_planes(pxp_solver_s *h, const double *delta, const double *beta, int 
   }
   h->medium_ok = false;
   h->cn_const = h->cn_vacuum = false;
+  cn_win_release(h, h->stream);
   free_dev(h->d_mat, h->stream);
   int rc;
   if ((rc = alloc(h, (void **)&h->d_mat, sizeof(double) * buf.size(), "material planes")))
@@ -1152,6 +1162,109 @@ int fft3d_variant(pxp_solver_s *h, const pxp::Fft3dPass &q0, const void *kx2, co
 
 bool cn_uses_const(const pxp_solver_s *h);
 
+// A medium sampled for enough steps, Dirichlet ends: steps solved with tables
+// factored ahead, alone and in batches.
+bool cn_uses_planes(const pxp_solver_s *h) {
+  return h->prob.kind == PXP_CRANK_NICHOLSON && !h->prob.transparent_bc && h->mat_stride != 0 &&
+         pxp::cn_planes_supported(pxp::cn_padded_n((int)h->nx), h->plane_count);
+}
+
+// Bytes a step of a window takes: its tables and the pivots they are made from.
+size_t cn_win_step_bytes(const pxp_solver_s *h) {
+  const int n = pxp::cn_padded_n((int)h->nx);
+  return pxp::cn_table_bytes(n) + pxp::cn_pivot_bytes(n);
+}
+
+// Steps of a buffer of at most `bytes`, for windows from `step` on.
+int cn_win_steps(const pxp_solver_s *h, long long step, size_t bytes) {
+  const size_t per = cn_win_step_bytes(h);
+  const long long left = (long long)h->plane_first + h->plane_count - step;
+  return (int)std::min<long long>(left, std::max<long long>(1, (long long)(bytes / per)));
+}
+
+// Whether the handle has a buffer for the tables of `step` and the steps after it
+// (they may still have to be computed); s: the stream that has used the
+// handle's buffer, or is ordered after it, and will use it next.
+bool cn_win_reserve(pxp_solver_s *h, long long step, size_t bytes, cudaStream_t s) {
+  const int cap = cn_win_steps(h, step, bytes);
+  const bool inside = step >= h->cn_win_first && step < (long long)h->cn_win_first + h->cn_win_count;
+  if (h->d_win != nullptr && (inside || h->cn_win_cap >= cap)) return true;
+  cn_win_release(h, s);
+  if (cudaMallocAsync((void **)&h->d_win, cap * cn_win_step_bytes(h), s) != cudaSuccess) {
+    cudaGetLastError();
+    h->d_win = nullptr;
+    return false;
+  }
+  h->cn_win_cap = cap;
+  return true;
+}
+
+// The part of a launch that takes the handle's steps from `step` on, at most
+// nsteps: in the window that holds `step`, or a new one in the same buffer.
+pxp::CnPlanes cn_win_part(pxp_solver_s *h, long long step, int nsteps) {
+  pxp::CnPlanes w{};
+  if (step < h->cn_win_first || step >= (long long)h->cn_win_first + h->cn_win_count) {
+    h->cn_win_first = (int)step;
+    h->cn_win_count = (int)std::min<long long>(h->cn_win_cap,
+                                               (long long)h->plane_first + h->plane_count - step);
+    w.factor = 1;
+  }
+  w.tabs = h->d_win;
+  w.pivots = h->d_win + h->cn_win_cap * pxp::cn_table_bytes(pxp::cn_padded_n((int)h->nx)) / sizeof(double2);
+  w.first = h->cn_win_first;
+  w.count = h->cn_win_count;
+  w.step0 = (int)step;
+  w.nsteps = (int)std::min<long long>(nsteps, (long long)w.first + w.count - step);
+  return w;
+}
+
+// At most this many bytes a handle.
+constexpr size_t kCnWindowBytes = size_t(96) << 20;
+
+// A solver's own steps.  The buffer stays with the handle while its window
+// holds steps to come; under stream capture the call brings its own, which the
+// captured work allocates and frees.
+cudaError_t cn_planes_steps(pxp_solver_s *h, long long first, int nsteps, int others) {
+  const int n = pxp::cn_padded_n((int)h->nx);
+  const bool flux = h->flux_count > 0;
+  const pxp::CnJob *job = (const pxp::CnJob *)h->d_job;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(h->stream, &cap);
+  if (e != cudaSuccess) return e;
+  const bool capturing = cap != cudaStreamCaptureStatusNone;
+  double2 *kept = nullptr;
+  int kept_cap = 0, kept_first = 0, kept_count = 0;
+  if (capturing) {
+    std::swap(kept, h->d_win);
+    std::swap(kept_cap, h->cn_win_cap);
+    std::swap(kept_first, h->cn_win_first);
+    std::swap(kept_count, h->cn_win_count);
+  }
+  int done = 0;
+  while (done < nsteps && e == cudaSuccess) {
+    const long long step = first + done;
+    if (!cn_win_reserve(h, step, kCnWindowBytes, h->stream)) {  // no memory: step by step
+      e = pxp::launch_cn(h->prec, job, 1, n, (int)step, nsteps - done, h->stream, flux);
+      break;
+    }
+    const pxp::CnPlanes w = cn_win_part(h, step, nsteps - done);
+    if (w.factor) e = pxp::launch_cn_factor(job, nullptr, w, 1, w.count, n, h->stream);
+    if (e == cudaSuccess)
+      e = pxp::launch_cn_planes(h->prec, job, nullptr, w, 1, n, h->stream, flux, others);
+    if (e != cudaSuccess) h->cn_win_count = 0;
+    done += w.nsteps;
+    if (first + done >= (long long)w.first + w.count) cn_win_release(h, h->stream);
+  }
+  if (capturing) {
+    cn_win_release(h, h->stream);
+    h->d_win = kept;
+    h->cn_win_cap = kept_cap;
+    h->cn_win_first = kept_first;
+    h->cn_win_count = kept_count;
+  }
+  return e;
+}
+
 // Handles of the process per device and dimension.  They may be stepping on
 // streams of their own beside a launch, which takes its size from them
 // (launch_cn_const); results never depend on it.
@@ -1530,6 +1643,7 @@ int pxp_solver_destroy(pxp_solver h) {
   free_dev(h->d_spheres, h->stream);
   free_dev(h->d_csg, h->stream);
   free_dev(h->d_lu, h->stream);
+  free_dev(h->d_win, h->stream);
   free_dev(h->d_ref, h->stream);
   free_dev(h->d_flux_win, h->stream);
   free_dev(h->d_flux, h->stream);
@@ -1836,6 +1950,7 @@ int pxp_set_initial_conditions(pxp_solver h, const double *field) {
   int rc = upload_field(h, h->d_field, field);
   if (rc) return rc;
   h->current_step = 1;
+  h->cn_win_count = 0;  // tables serve one pass through the medium
   h->ic_set = true;
   return PXP_OK;
 }
@@ -1845,6 +1960,7 @@ int pxp_set_initial_conditions_device(pxp_solver h, const void *dfield) {
   PXP_TRY_CUDA(h, cudaMemcpyAsync(h->d_field, dfield, h->csize * h->npts,
                                   cudaMemcpyDeviceToDevice, h->stream));
   h->current_step = 1;
+  h->cn_win_count = 0;
   h->ic_set = true;
   return PXP_OK;
 }
@@ -1881,12 +1997,9 @@ int pxp_step(pxp_solver h, int nsteps) {
                                  h->flux_count > 0, sms_of_others(h->prob.device, 1));
         break;
       }
-      e = cudaErrorMemoryAllocation;
-      if (!h->prob.transparent_bc && pxp::cn_planes_supported(pxp::cn_padded_n((int)h->nx), nsteps))
-        e = pxp::launch_cn_planes(h->prec, (const pxp::CnJob *)h->d_job,
-                                  pxp::cn_padded_n((int)h->nx), (int)first, nsteps, h->stream,
-                                  h->flux_count > 0);
-      if (e == cudaErrorMemoryAllocation)
+      if (cn_uses_planes(h))
+        e = cn_planes_steps(h, first, nsteps, sms_of_others(h->prob.device, 1));
+      else
         e = pxp::launch_cn(h->prec, (const pxp::CnJob *)h->d_job, 1,
                            pxp::cn_padded_n((int)h->nx), (int)first, nsteps, h->stream,
                            h->flux_count > 0);
@@ -2482,6 +2595,39 @@ bool cn_uses_const(const pxp_solver_s *h) {
   return h->cn_const && !h->prob.transparent_bc && h->mat_stride == 0;
 }
 
+// A batch's windows of sampled media, all jobs together.
+constexpr size_t kCnBatchBytes = size_t(12) << 30;
+
+// A launch of a group of sampled-media jobs: every job's part of it.
+struct CnPart {
+  std::vector<pxp::CnPlanes> list;
+  int factor_steps = 0;  // the largest window to factor
+  size_t offset = 0;     // of the list in the batch's job array
+};
+
+std::vector<CnPart> cn_batch_parts(const std::vector<pxp_solver_s *> &jobs, int max_steps) {
+  std::vector<CnPart> out;
+  std::vector<int> done(jobs.size(), 0);
+  for (bool more = true; more;) {
+    more = false;
+    CnPart c;
+    for (size_t i = 0; i < jobs.size(); ++i) {
+      pxp_solver_s *h = jobs[i];
+      const int left = std::min(h->batch_remaining, max_steps) - done[i];
+      pxp::CnPlanes w{};
+      if (left > 0) {
+        w = cn_win_part(h, (long long)h->current_step + done[i], left);
+        done[i] += w.nsteps;
+        more = true;
+        if (w.factor) c.factor_steps = std::max(c.factor_steps, w.count);
+      }
+      c.list.push_back(w);
+    }
+    if (more) out.push_back(std::move(c));
+  }
+  return out;
+}
+
 int grow(pxp_batch_s *b, size_t bytes) {
   if (bytes <= b->d_jobs_cap) return PXP_OK;
   size_t cap = std::max(bytes, 2 * b->d_jobs_cap);
@@ -2573,7 +2719,8 @@ int pxp_batch_round(pxp_batch b, int max_steps) {
       if (int rc = check_medium(h)) return b->fail(rc, h->err);
   // the staging buffer of the previous round must be consumed
   if (cudaStreamSynchronize(b->stream) != cudaSuccess) return b->fail(PXP_ERR_CUDA, "batch stream");
-  // ---- 2-D groups: key (kind, n, precision, CN matrix path)
+  // ---- 2-D groups: key (kind, n, precision, CN path: 0 step by step, 1 a
+  // step-invariant matrix, 2 tables of sampled media, the paths of pxp_step)
   struct Key {
     int kind, n, prec, cpath;
     bool operator<(const Key &o) const {
@@ -2581,9 +2728,15 @@ int pxp_batch_round(pxp_batch b, int max_steps) {
     }
   };
   std::map<Key, std::vector<pxp_solver_s *>> groups;
+  size_t sampled = 0;
+  for (const pxp_solver_s *h : b->active) sampled += h->batch_remaining > 0 && cn_uses_planes(h);
   for (pxp_solver_s *h : b->active) {
     if (!is_2d(h) || h->batch_remaining <= 0) continue;
-    Key k{h->prob.kind, (int)h->nx, (int)h->prec, h->prob.kind == PXP_CRANK_NICHOLSON ? (int)cn_uses_const(h) : 0};
+    Key k{h->prob.kind, (int)h->nx, (int)h->prec, 0};
+    if (h->prob.kind == PXP_CRANK_NICHOLSON && cn_uses_const(h)) k.cpath = 1;
+    if (cn_uses_planes(h) &&
+        cn_win_reserve(h, h->current_step, std::min(kCnWindowBytes, kCnBatchBytes / sampled), b->stream))
+      k.cpath = 2;
     groups[k].push_back(h);
   }
   // Within a group the CTA index follows the job order, and the block
@@ -2597,7 +2750,24 @@ int pxp_batch_round(pxp_batch b, int max_steps) {
                        return std::min(a->batch_remaining, max_steps) >
                               std::min(c->batch_remaining, max_steps);
                      });
+  // sampled media: each group's launches, every job's next window or the rest of
+  // one in each
+  std::map<Key, std::vector<CnPart>> parts;
+  // windows planned in the handles hold nothing before their launch: a round that
+  // fails earlier drops them
+  struct Planned {
+    std::vector<pxp_solver_s *> jobs;
+    ~Planned() {
+      for (pxp_solver_s *h : jobs) h->cn_win_count = 0;
+    }
+  } planned;
+  for (auto &g : groups)
+    if (g.first.cpath == 2) {
+      parts[g.first] = cn_batch_parts(g.second, max_steps);
+      planned.jobs.insert(planned.jobs.end(), g.second.begin(), g.second.end());
+    }
   size_t total = 0;
+  for (auto &g : parts) total += g.second.size() * groups[g.first].size() * sizeof(pxp::CnPlanes);
   for (auto &g : groups)
     total += g.second.size() * (g.first.kind == PXP_FFT_SOLVER_2D ? sizeof(pxp::Fft1dJob) : sizeof(pxp::CnJob));
   if (total > 0) {
@@ -2605,6 +2775,12 @@ int pxp_batch_round(pxp_batch b, int max_steps) {
     if (rc) return rc;
   }
   size_t off = 0;
+  for (auto &g : parts)
+    for (CnPart &c : g.second) {
+      c.offset = off;
+      std::memcpy((char *)b->h_jobs + off, c.list.data(), sizeof(pxp::CnPlanes) * c.list.size());
+      off += sizeof(pxp::CnPlanes) * c.list.size();
+    }
   std::vector<std::pair<size_t, const std::pair<const Key, std::vector<pxp_solver_s *>> *>> offs;
   for (auto &g : groups) {
     offs.push_back({off, &g});
@@ -2675,10 +2851,29 @@ int pxp_batch_round(pxp_batch b, int max_steps) {
         e = pxp::launch_fft1d((pxp::Precision)k.prec, (const pxp::Fft1dJob *)jobs,
                               (int)list.size(), k.n, -1, -1, gst, any_flux, b->d_queue + gi);
     }
-    else if (k.cpath)
+    else if (k.cpath == 1)
       e = pxp::launch_cn_const((pxp::Precision)k.prec, (const pxp::CnJob *)jobs, (int)list.size(),
                                pxp::cn_padded_n(k.n), -1, -1, gst, any_flux,
                                sms_of_others(b->device, (int)list.size()));
+    else if (k.cpath == 2) {
+      const int n = pxp::cn_padded_n(k.n), nj = (int)list.size();
+      e = cudaSuccess;
+      for (const CnPart &c : parts[k]) {
+        const pxp::CnPlanes *d_list = (const pxp::CnPlanes *)((const char *)b->d_jobs + c.offset);
+        if (e == cudaSuccess)
+          e = pxp::launch_cn_factor((const pxp::CnJob *)jobs, d_list, pxp::CnPlanes{}, nj, c.factor_steps, n,
+                                    gst);
+        if (e == cudaSuccess)
+          e = pxp::launch_cn_planes((pxp::Precision)k.prec, (const pxp::CnJob *)jobs, d_list,
+                                    pxp::CnPlanes{}, nj, n, gst, any_flux, sms_of_others(b->device, nj));
+      }
+      if (e == cudaSuccess)
+        for (pxp_solver_s *h : list) {
+          planned.jobs.erase(std::find(planned.jobs.begin(), planned.jobs.end(), h));
+          const long long next = (long long)h->current_step + std::min(h->batch_remaining, max_steps);
+          if (next >= (long long)h->cn_win_first + h->cn_win_count) cn_win_release(h, gst);
+        }
+    }
     else
       e = pxp::launch_cn((pxp::Precision)k.prec, (const pxp::CnJob *)jobs, (int)list.size(),
                          pxp::cn_padded_n(k.n), -1, -1, gst, any_flux);

@@ -6,10 +6,10 @@
 // (or a cluster) owns one problem; the field stays on chip for every step of
 // the launch.  Three kernels:
 //   cn_const_kernel   z-invariant media, Dirichlet ends;
-//   cn_planes_kernel  media sampled per step, Dirichlet ends, a block of steps
-//                     factored ahead by cn_factor_kernel;
-//   cn_kernel         everything else (transparent ends, short calls, batches
-//                     of sampled media), step by step:
+//   cn_planes_kernel  media sampled per step, Dirichlet ends, a window of steps
+//                     factored ahead by cn_pivot_kernel and cn_table_kernel;
+//   cn_kernel         everything else (transparent ends, media sampled for few
+//                     steps), step by step:
 //   1. each thread builds the matrix rows of its chunk of M consecutive points
 //      (diag, rhs; sub-diagonal constant) with the reference's operation
 //      order, rounded op by op, so the coefficients equal the reference's;
@@ -496,9 +496,10 @@ __global__ void __launch_bounds__(T) cn_const_kernel(const CnJob *__restrict__ j
 }
 
 // Media sampled per step: every step has its own matrix, but none depends on
-// the field, so the pivots of a block of steps are computed ahead, a CTA a
-// step on as many SMs (cn_factor_kernel), and the sequential kernel
-// (cn_planes_kernel) only solves with them.
+// the field, so a window of steps is factored ahead (cn_pivot_kernel,
+// cn_table_kernel) and the sequential kernel (cn_planes_kernel) only solves with
+// its tables.  A launch takes a list of problems (CnPlanes); every problem's
+// arithmetic is the same alone and among others, and whatever the windows.
 //
 // Tables of a step: [c | hL | hR | w], c = 2 + m - m', rows in the solving
 // kernel's order (row m of thread tt at m*TT + tt, TT threads over the
@@ -548,60 +549,114 @@ __device__ __forceinline__ PivotInv pivot_inverse(double2 b, QSq q2, PivotInv pr
   return {r, cmul(r, mk(rx, ry))};
 }
 
-// The two pivot recurrences are serial (two threads a step, some 200 cycles a
-// row), which a block of steps hides; everything else is parallel over rows.
-template <int M, int TT>
-__global__ void __launch_bounds__(TT < 64 ? 64 : TT)
-    cn_factor_kernel(const CnJob *__restrict__ jobs, double2 *__restrict__ tabs, int step0) {
-  constexpr int NP = M * TT, TW = TT / 32, T = TT < 64 ? 64 : TT;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2 *pl = reinterpret_cast<double2 *>(smem_raw);  // b, then 1/pivot from the left
-  double2 *pr = pl + NP;                                // the same from the right
-  double2 *tot = pr + NP;                               // 2 x TW
-  float2 *ll = reinterpret_cast<float2 *>(tot + 2 * TW);  // their second words
-  float2 *lr = ll + NP;
-  const CnJob job = jobs[0];
-  const int t = threadIdx.x, n = job.n_real > 0 ? job.n_real : NP;
-  const int step = step0 + (int)blockIdx.x;
-  const long long off = job.mat_stride * (long long)(step - job.mat_step0);
-  const double *de = job.delta + off, *be = job.beta + off;
-  for (int i = t; i < NP; i += T) {
-    // the padding rows' pivots are kCnPad
-    pl[i] = pr[i] = i < n ? cn_diag(de[i], be[i], job.rho, job.r) : mk(1.0 / kCnPad, 0.0);
-    ll[i] = lr[i] = make_float2(0.f, 0.f);
+// Pivots of one recurrence of a step: row k (from the left, or DIR < 0 from the
+// right) from de[k * DIR] and be[k * DIR] to hi[k * DIR] and lo[k * DIR].
+template <int DIR>
+__device__ __forceinline__ void pivot_chain(const double *__restrict__ de, const double *__restrict__ be,
+                                            double2 *__restrict__ hi, float2 *__restrict__ lo, int n,
+                                            double rho, double r) {
+  const double q = 0.25 * rho;
+  QSq q2;
+  q2.hi = __dmul_rn(q, q);
+  q2.lo = __fma_rn(q, q, -q2.hi);
+  PivotInv inv = {mk(0.0, 0.0), mk(0.0, 0.0)};
+  auto row = [&](int k, double d, double b) {
+    inv = pivot_inverse(cn_diag(d, b, rho, r), q2, inv);
+    hi[k * DIR] = inv.hi;
+    lo[k * DIR] = make_float2((float)inv.lo.x, (float)inv.lo.y);
+  };
+  // whole groups of rows, each group's inputs loaded while the one before is
+  // worked on
+  constexpr int U = 8;
+  double dn[U], bn[U];
+  const int full = n / U;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    dn[u] = full > 0 ? de[u * DIR] : 0.0;
+    bn[u] = full > 0 ? be[u * DIR] : 0.0;
   }
-  __syncthreads();
+#pragma unroll 1
+  for (int g = 0; g < full; ++g) {
+    double d[U], b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      d[u] = dn[u];
+      b[u] = bn[u];
+    }
+    const int next = g + 1 < full ? U : 0;  // the last group loads itself again
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      dn[u] = de[(next + u) * DIR];
+      bn[u] = be[(next + u) * DIR];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) row(u, d[u], b[u]);
+    de += U * DIR;
+    be += U * DIR;
+    hi += U * DIR;
+    lo += U * DIR;
+  }
+#pragma unroll 1
+  for (int k = 0; k < n - full * U; ++k) row(k, de[k * DIR], be[k * DIR]);
+}
+
+// The pivots of a window's steps: the two recurrences of a step are serial (some
+// 130 ns a row), so a thread takes one of them and a warp 32 steps'; a window of
+// a few hundred steps then needs some twenty warps, and problems stepping side by
+// side share the SMs.  Pivot i of step st and direction d goes to workspace
+// entry (2 st + d) * np + i, second words after the first ones.
+__global__ void __launch_bounds__(32)
+    cn_pivot_kernel(const CnJob *__restrict__ jobs, const CnPlanes *__restrict__ list, const CnPlanes one,
+                    int np) {
+  const CnPlanes w = list ? list[blockIdx.y] : one;
+  const int dir = blockIdx.x & 1, st = (blockIdx.x >> 1) * 32 + threadIdx.x;
+  if (!w.factor || st >= w.count) return;
+  const CnJob &job = jobs[blockIdx.y];
+  const int n = job.n_real > 0 ? job.n_real : np;
+  const long long off = job.mat_stride * (long long)(w.first + st - job.mat_step0);
+  const double *de = job.delta + off, *be = job.beta + off;
+  const size_t at = (size_t)(2 * st + dir) * np;
+  double2 *hi = w.pivots + at;
+  float2 *lo = reinterpret_cast<float2 *>(w.pivots + 2 * (size_t)w.count * np) + at;
+  if (dir == 0) pivot_chain<1>(de, be, hi, lo, n, job.rho, job.r);
+  else pivot_chain<-1>(de + n - 1, be + n - 1, hi + n - 1, lo + n - 1, n, job.rho, job.r);
+}
+
+// The tables of a window's steps from its pivots, a CTA a step; everything here
+// is parallel over rows.
+template <int M, int TT>
+__global__ void __launch_bounds__(TT)
+    cn_table_kernel(const CnJob *__restrict__ jobs, const CnPlanes *__restrict__ list, const CnPlanes one) {
+  constexpr int NP = M * TT, TW = TT / 32;
+  __shared__ double2 tot[2 * TW];
+  const CnPlanes pw = list ? list[blockIdx.y] : one;
+  const int st = blockIdx.x;
+  if (!pw.factor || st >= pw.count) return;
+  const CnJob job = jobs[blockIdx.y];
+  const int t = threadIdx.x, n = job.n_real > 0 ? job.n_real : NP;
+  const long long off = job.mat_stride * (long long)(pw.first + st - job.mat_step0);
+  const double *de = job.delta + off, *be = job.beta + off;
+  const double *dp = job.delta_prev + off, *bp = job.beta_prev + off;
+  const double2 *hi = pw.pivots + (size_t)(2 * st) * NP;
+  const float2 *lo =
+      reinterpret_cast<const float2 *>(pw.pivots + 2 * (size_t)pw.count * NP) + (size_t)(2 * st) * NP;
+  // the padding rows' pivots are kCnPad; beyond the system there is none
+  auto pivot = [&](int dir, int i) {
+    const double2 zero = mk(0.0, 0.0);
+    if (i < 0 || i >= NP) return PivotInv{zero, zero};
+    if (i >= n) return PivotInv{mk(1.0 / kCnPad, 0.0), zero};
+    return PivotInv{hi[dir * NP + i], to_d(lo[dir * NP + i])};
+  };
   const double q = 0.25 * job.rho;
   QSq q2;
   q2.hi = __dmul_rn(q, q);
   q2.lo = __fma_rn(q, q, -q2.hi);
-  if (t == 0 || t == 32) {
-    double2 *pv = t == 0 ? pl : pr;
-    float2 *lo = t == 0 ? ll : lr;
-    const int first = t == 0 ? 0 : n - 1, by = t == 0 ? 1 : -1;
-    PivotInv inv = {mk(0.0, 0.0), mk(0.0, 0.0)};
-    double2 b = pv[first];
-#pragma unroll 2
-    for (int k = 0; k < n; ++k) {
-      const int i = first + k * by;
-      const double2 nb = k + 1 < n ? pv[i + by] : b;
-      inv = pivot_inverse(b, q2, inv);
-      pv[i] = inv.hi;
-      lo[i] = make_float2((float)inv.lo.x, (float)inv.lo.y);
-      b = nb;
-    }
-  }
-  __syncthreads();
-  if (T > TT && t >= TT) return;  // no barrier follows for a single warp of rows
-  double2 *out = tabs + blockIdx.x * cn_step_entries(M, TT);
-  const double *dp = job.delta_prev + off, *bp = job.beta_prev + off;
+  double2 *out = pw.tabs + st * cn_step_entries(M, TT);
   double2 aL = mk(1.0, 0.0), aR = mk(1.0, 0.0);
 #pragma unroll
   for (int m = 0; m < M; ++m) {
     const int i = t * M + m;
-    const double2 zero = mk(0.0, 0.0);
-    const PivotInv il = i > 0 ? PivotInv{pl[i - 1], to_d(ll[i - 1])} : PivotInv{zero, zero};
-    const PivotInv ir = i < NP - 1 ? PivotInv{pr[i + 1], to_d(lr[i + 1])} : PivotInv{zero, zero};
+    const PivotInv il = pivot(0, i - 1), ir = pivot(1, i + 1);
     const double2 hL = mk(-fma(q, il.hi.y, q * il.lo.y), fma(q, il.hi.x, q * il.lo.x));
     const double2 hR = mk(-fma(q, ir.hi.y, q * ir.lo.y), fma(q, ir.hi.x, q * ir.lo.x));
     double2 c = mk(2.0, 0.0), b = mk(kCnPad, 0.0);
@@ -651,33 +706,44 @@ template <int N> __device__ __forceinline__ void cn_cp_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// The steps of a block with the tables above.  Every thread copies its own
+constexpr bool cn_c_in_registers(int M, int T) { return M * T > 1024; }
+
+// The steps of a window with the tables above.  Every thread copies its own
 // table entries a step ahead into slots of its own (no barrier): hL and hR,
 // used until the carries are folded in, into alternating buffers, the others
 // into the slots just read.  Four copy groups a step, in the order they are
-// used: {hL, hR}, {c}, {products}, {w}.
-// What bounds it: the const kernel's chains plus the tables' way from L2 (78
-// bytes a row and step into its SMs), and the pivot chains (2048 rows: some 0.5
-// ms a block).  Measured over 300 steps, us a step, before (chunk elimination
-// and cyclic reduction of every step's matrix in turn, cn_kernel): 300 rows 9.3 ->
-// 2.3, 1000: 11.7 -> 3.2, 3000: 25.7 -> 8.7; 1501 rows, 400 steps 15.6 -> 6.7;
-// FP32 700: 10.3 -> 3.1.  Errors against an 80-bit sweep, 1501 and 3000 rows:
-// 2e-13 and 2e-12 -> 0.05 .. 0.2e-12 and 0.04 .. 0.6e-12 (with pivots of one
-// word 1.4e-12 and 2.2e-12).
+// used: {hL, hR}, {c}, {products}, {w}.  With 2048 rows a CTA there is no room
+// for c, which waits in registers (slower elsewhere: 200 rows, 400 steps 719
+// against 590 us).
+// What bounds it: the const kernel's chains plus the tables' way from L2 (92
+// bytes a row and step into its SMs), and the pivot chains in front of every
+// window.  Measured, us a step and us of pivots a window (step by step,
+// cn_kernel): 300 rows 1.0 and 75 (8.2), 1000: 1.2 and 157 (10.8), 1501: 1.9 and
+// 218 (15.1), 4000: 1.9 and 513 (27); eight problems of 1501 rows and 200 steps
+// in a batch 0.91 ms (3.17), 40 of them 2.1 (3.7), 148, whose 11 GB of pivots
+// and tables go through HBM, 9.7 (5.6).  Errors against an 80-bit sweep, 1501
+// and 3000 rows: 0.05 .. 0.2e-12 and 0.04 .. 0.6e-12 (step by step 2e-13 and
+// 2e-12; with pivots of one word 1.4e-12 and 2.2e-12).
 template <typename R, int M, int T, int K, bool FLUX>
 __global__ void __launch_bounds__(T) cn_planes_kernel(const CnJob *__restrict__ jobs,
-                                                     const double2 *__restrict__ tabs, int step0,
-                                                     int nsteps) {
+                                                     const CnPlanes *__restrict__ list,
+                                                     const CnPlanes one) {
   using C = typename Cx<R>::T;
   constexpr int NC = M * T, W = T / 32, TW = W * K, TT = T * K;
+  constexpr bool CREG = cn_c_in_registers(M, T);
+  constexpr int AHEAD = CREG ? 2 : 3;  // groups younger than the one to wait for
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2 *sH = reinterpret_cast<double2 *>(smem_raw);  // 2 x [hL | hR]
   double2 *sC = sH + 4 * NC;
-  double2 *sW = sC + NC;
-  double2 *sP = sW + NC;            // 14 x T
+  double2 *sW = CREG ? sC : sC + NC;
+  double2 *sP = sW + NC;             // 14 x T
   double2 *tot = sP + kCnCoefs * T;  // 2 x 2 x TW
   __shared__ double flux_part[2][TW];
-  const CnJob job = jobs[0];
+  const CnPlanes pw = list ? list[blockIdx.x / K] : one;
+  const int step0 = pw.step0, nsteps = pw.nsteps;
+  if (nsteps <= 0) return;  // the whole cluster
+  const CnJob job = jobs[blockIdx.x / K];
+  const double2 *tabs = pw.tabs + (step0 - pw.first) * cn_step_entries(M, T * K);
   const int t = threadIdx.x, rank = K > 1 ? (int)(blockIdx.x % K) : 0;
   const int gw = rank * W + t / 32, tt = rank * T + t;
   const int s0 = tt * M;
@@ -695,7 +761,16 @@ __global__ void __launch_bounds__(T) cn_planes_kernel(const CnJob *__restrict__ 
     fetch(st, 2, dst + NC, M);
     cn_cp_commit();
   };
-  auto fetch_c = [&](int st) { fetch(st, 0, sC, M); cn_cp_commit(); };
+  double2 c[CREG ? M : 1];
+  auto fetch_c = [&](int st) {
+    if constexpr (!CREG) {
+      fetch(st, 0, sC, M);
+      cn_cp_commit();
+    } else if (st < nsteps) {
+#pragma unroll
+      for (int m = 0; m < M; ++m) c[m] = __ldg(tabs + st * cn_step_entries(M, TT) + (size_t)m * TT + tt);
+    }
+  };
   auto fetch_p = [&](int st) { fetch(st, 4, sP, kCnCoefs); cn_cp_commit(); };
   auto fetch_w = [&](int st) { fetch(st, 3, sW, M); cn_cp_commit(); };
   fetch_h(0);
@@ -730,13 +805,13 @@ __global__ void __launch_bounds__(T) cn_planes_kernel(const CnJob *__restrict__ 
     const double2 *hl = sH + (st & 1) * 2 * NC + t, *hr = hl + NC;
     double2 x[M];
 #pragma unroll
-    for (int m = 0; m < M; ++m) x[m] = cmul(sC[m * T + t], u[m]);
+    for (int m = 0; m < M; ++m) x[m] = cmul(CREG ? c[m] : sC[m * T + t], u[m]);
     fetch_c(st + 1);
     two_sided_solve<M, TW>(
         x, [&](int m) { return hl[m * T]; }, [&](int m) { return hr[m * T]; },
         [&](int m) { return sW[m * T + t]; },
         [&] {
-          cn_cp_wait<3>();
+          cn_cp_wait<AHEAD>();
           ScanCoef c;
 #pragma unroll
           for (int k = 0; k < 5; ++k) {
@@ -751,7 +826,7 @@ __global__ void __launch_bounds__(T) cn_planes_kernel(const CnJob *__restrict__ 
         },
         tot + par * 2 * TW, gw, publish, sync, [&] {
           fetch_p(st + 1);
-          cn_cp_wait<3>();  // {w}
+          cn_cp_wait<AHEAD>();  // {w}
         });
     fetch_w(st + 1);
     const double acc = cn_finish<R>(job, step, u, x, s0, nreal, flux, fw);
@@ -812,15 +887,16 @@ bool cn_const_supported(Precision, int n) {
 // step against 22.9.)  The forms have the same chunks and warps and give the
 // same bits.  2048 rows gain too little (1.40 on one SM, 1.31 on two).
 constexpr int kSms = 148;
+static bool cn_wide(int nj, int ctas, int others) {
+  // PXP_CN_CLUSTER=0|1 pins the narrowest or the widest form
+  const char *pin = std::getenv("PXP_CN_CLUSTER");
+  if (pin && (pin[0] == '0' || pin[0] == '1')) return pin[0] == '1';
+  return (long long)nj * ctas + others <= kSms;
+}
 cudaError_t launch_cn_const(Precision p, const CnJob *d_jobs, int nj, int n, int step0, int nsteps,
                             cudaStream_t s, bool flux, int others) {
   if (nj <= 0) return cudaSuccess;
-  // PXP_CN_CLUSTER=0|1 pins the narrowest or the widest form
-  const char *pin = std::getenv("PXP_CN_CLUSTER");
-  auto wide = [&](int ctas) {
-    if (pin && (pin[0] == '0' || pin[0] == '1')) return pin[0] == '1';
-    return (long long)nj * ctas + others <= kSms;
-  };
+  auto wide = [&](int ctas) { return cn_wide(nj, ctas, others); };
 #define PXP_CT(MM, TT, KK)                                                                \
   p == kFP64 ? cn_const_launch_t<double, MM, TT, KK>(d_jobs, nj, step0, nsteps, s, flux) \
              : cn_const_launch_t<float, MM, TT, KK>(d_jobs, nj, step0, nsteps, s, flux)
@@ -839,58 +915,73 @@ cudaError_t launch_cn_const(Precision p, const CnJob *d_jobs, int nj, int n, int
 #undef PXP_CT
 }
 
+template <int M, int TT>
+static cudaError_t cn_factor_launch_t(const CnJob *d_jobs, const CnPlanes *d_list, const CnPlanes &one,
+                                      int nj, int count, cudaStream_t s) {
+  cn_pivot_kernel<<<dim3(2 * ((count + 31) / 32), nj), 32, 0, s>>>(d_jobs, d_list, one, M * TT);
+  cn_table_kernel<M, TT><<<dim3(count, nj), TT, 0, s>>>(d_jobs, d_list, one);
+  return cudaGetLastError();
+}
+
 template <typename R, int M, int T, int K>
-static cudaError_t cn_planes_launch_t(const CnJob *d_job, int step0, int nsteps, cudaStream_t s,
-                                      bool flux) {
-  constexpr int TT = T * K;
-  constexpr size_t fsm = sizeof(double2) * (3 * M * TT + 2 * (TT / 32));
-  constexpr size_t psm = sizeof(double2) * (6 * M * T + kCnCoefs * T + 4 * (TT / 32));
-  static_assert(fsm <= 227 * 1024 && psm <= 226 * 1024, "tables exceed shared memory");
-  auto kf = cn_factor_kernel<M, TT>;
-  cudaError_t e = raise_dynamic_smem((const void *)kf, (int)fsm);
-  if (e != cudaSuccess) return e;
-  constexpr size_t per = sizeof(double2) * cn_step_entries(M, TT);
-  // a block of steps: at most 64 MB of tables
-  const int block = (int)std::min<size_t>((size_t)nsteps, (size_t(64) << 20) / per);
-  double2 *tabs = nullptr;
-  e = cudaMallocAsync((void **)&tabs, per * block, s);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return cudaErrorMemoryAllocation;
-  }
-  for (int i = 0; i < nsteps && e == cudaSuccess; i += block) {
-    const int k = std::min(block, nsteps - i);
-    kf<<<k, TT < 64 ? 64 : TT, fsm, s>>>(d_job, tabs, step0 + i);
-    e = cudaGetLastError();
-    if (e == cudaSuccess)
-      e = flux ? cn_cluster_launch(cn_planes_kernel<R, M, T, K, true>, K, K, T, psm, s, d_job,
-                                   (const double2 *)tabs, step0 + i, k)
-               : cn_cluster_launch(cn_planes_kernel<R, M, T, K, false>, K, K, T, psm, s, d_job,
-                                   (const double2 *)tabs, step0 + i, k);
-  }
-  const cudaError_t f = cudaFreeAsync(tabs, s);
-  if (e == cudaSuccess) e = f;
-  // that code means that nothing ran
-  return e == cudaErrorMemoryAllocation ? cudaErrorLaunchFailure : e;
+static cudaError_t cn_planes_launch_t(const CnJob *d_jobs, const CnPlanes *d_list, const CnPlanes &one,
+                                      int nj, cudaStream_t s, bool flux) {
+  constexpr size_t smem =
+      sizeof(double2) * ((cn_c_in_registers(M, T) ? 5 : 6) * M * T + kCnCoefs * T + 4 * (T / 32) * K);
+  static_assert(smem <= 226 * 1024, "tables exceed shared memory");
+  return flux ? cn_cluster_launch(cn_planes_kernel<R, M, T, K, true>, nj * K, K, T, smem, s, d_jobs, d_list,
+                                  one)
+              : cn_cluster_launch(cn_planes_kernel<R, M, T, K, false>, nj * K, K, T, smem, s, d_jobs, d_list,
+                                  one);
 }
 
-// Below some 20 steps a call the pivot chains cost more than they save (1501
-// rows: 16 steps 346 against 368 us with cn_kernel, 8 steps 319 against 245).
-bool cn_planes_supported(int n, int nsteps) {
-  return n >= 64 && n <= 4096 && nsteps >= 24;
-}
+// By the medium, not by a call's steps, so that a problem takes one path
+// however its steps are split.  Below some 20 steps the pivots cost more than
+// the faster steps save (us for 16 and 24 steps in one call, step by step and
+// here: 100 rows 98, 137 and 56, 64; 300: 150, 215 and 90, 98; 1000: 194, 280 and
+// 177, 186; 1501: 262, 383 and 249, 264; 4000: 456, 672 and 545, 559).
+bool cn_planes_supported(int n, int planes) { return n >= 64 && n <= 4096 && planes >= 24; }
 
-cudaError_t launch_cn_planes(Precision p, const CnJob *d_job, int n, int step0, int nsteps,
-                             cudaStream_t s, bool flux) {
-#define PXP_CP(NN, MM, TT, KK)                                                                \
-  case NN:                                                                                    \
-    return p == kFP64 ? cn_planes_launch_t<double, MM, TT, KK>(d_job, step0, nsteps, s, flux) \
-                      : cn_planes_launch_t<float, MM, TT, KK>(d_job, step0, nsteps, s, flux);
+// Chunk and threads of a problem of n padded rows (64 .. 4096).
+static void cn_planes_shape(int n, int *m, int *tt) {
+  *tt = n < 256 ? 32 : n / 8;
+  *m = n / *tt;
+}
+size_t cn_table_bytes(int n) {
+  int m, tt;
+  cn_planes_shape(n, &m, &tt);
+  return sizeof(double2) * cn_step_entries(m, tt);
+}
+size_t cn_pivot_bytes(int n) { return 2 * (sizeof(double2) + sizeof(float2)) * (size_t)n; }
+
+cudaError_t launch_cn_factor(const CnJob *d_jobs, const CnPlanes *d_list, const CnPlanes &one, int nj,
+                             int count, int n, cudaStream_t s) {
+  if (nj <= 0 || count <= 0) return cudaSuccess;
+#define PXP_CF(NN, MM, TT) case NN: return cn_factor_launch_t<MM, TT>(d_jobs, d_list, one, nj, count, s);
   switch (n) {
-    PXP_CP(64, 2, 32, 1) PXP_CP(128, 4, 32, 1) PXP_CP(256, 8, 32, 1) PXP_CP(512, 8, 64, 1)
-    PXP_CP(1024, 8, 128, 1) PXP_CP(2048, 8, 128, 2) PXP_CP(4096, 8, 128, 4)
-    default:
-      return cudaErrorInvalidValue;
+    PXP_CF(64, 2, 32) PXP_CF(128, 4, 32) PXP_CF(256, 8, 32) PXP_CF(512, 8, 64) PXP_CF(1024, 8, 128)
+    PXP_CF(2048, 8, 256) PXP_CF(4096, 8, 512)
+    default: return cudaErrorInvalidValue;
+  }
+#undef PXP_CF
+}
+
+// CTAs a problem by the same rule as launch_cn_const's.
+cudaError_t launch_cn_planes(Precision p, const CnJob *d_jobs, const CnPlanes *d_list, const CnPlanes &one,
+                             int nj, int n, cudaStream_t s, bool flux, int others) {
+  if (nj <= 0) return cudaSuccess;
+#define PXP_CP(MM, TT, KK)                                                                  \
+  p == kFP64 ? cn_planes_launch_t<double, MM, TT, KK>(d_jobs, d_list, one, nj, s, flux)     \
+             : cn_planes_launch_t<float, MM, TT, KK>(d_jobs, d_list, one, nj, s, flux)
+  switch (n) {
+    case 64: return PXP_CP(2, 32, 1);
+    case 128: return PXP_CP(4, 32, 1);
+    case 256: return PXP_CP(8, 32, 1);
+    case 512: return PXP_CP(8, 64, 1);
+    case 1024: return PXP_CP(8, 128, 1);
+    case 2048: return cn_wide(nj, 2, others) ? PXP_CP(8, 128, 2) : PXP_CP(8, 256, 1);
+    case 4096: return cn_wide(nj, 4, others) ? PXP_CP(8, 128, 4) : PXP_CP(8, 256, 2);
+    default: return cudaErrorInvalidValue;
   }
 #undef PXP_CP
 }

@@ -131,13 +131,26 @@ constexpr double kCnPad = 1e30;
 cudaError_t launch_cn_const(Precision p, const CnJob *d_jobs, int nj, int n, int step0,
                             int nsteps, cudaStream_t s, bool flux, int others);
 bool cn_const_supported(Precision p, int n);
-// Media sampled per step, Dirichlet ends: the matrices of a block of steps are
-// factored ahead on all SMs (workspace from the stream's pool).  Worth it from
-// some steps a call on; cudaErrorMemoryAllocation (nothing launched) when the
-// workspace cannot be had: launch_cn then.
-bool cn_planes_supported(int n, int nsteps);
-cudaError_t launch_cn_planes(Precision p, const CnJob *d_job, int n, int step0, int nsteps,
-                             cudaStream_t s, bool flux);
+// Media sampled per step, Dirichlet ends, for n padded rows and a medium of
+// `planes` steps: the matrices of a window of steps are factored ahead
+// (launch_cn_factor) and the steps solved with their tables (launch_cn_planes).
+// One problem's part of such a launch:
+struct CnPlanes {
+  double2 *tabs;      // the tables of the window's steps (cn_table_bytes each)
+  double2 *pivots;    // workspace of its factoring (cn_pivot_bytes a step)
+  int first, count;   // the window: its first step, its steps
+  int factor;         // whether its tables are to be computed
+  int step0, nsteps;  // the steps to solve, inside the window (may be none)
+};
+bool cn_planes_supported(int n, int planes);
+size_t cn_table_bytes(int n);
+size_t cn_pivot_bytes(int n);
+// nj problems, each with its job and its entry of d_list (null: one problem,
+// `one`); count: the largest window to factor.  others as for launch_cn_const.
+cudaError_t launch_cn_factor(const CnJob *d_jobs, const CnPlanes *d_list, const CnPlanes &one, int nj,
+                             int count, int n, cudaStream_t s);
+cudaError_t launch_cn_planes(Precision p, const CnJob *d_jobs, const CnPlanes *d_list, const CnPlanes &one,
+                             int nj, int n, cudaStream_t s, bool flux, int others);
 
 // ------------------------------------------------------------- ADI ------
 struct Sphere {

@@ -4,13 +4,15 @@
 // launch is only counted.  fake_fail_allocations(k) makes the k-th
 // cudaMallocAsync from then on fail, and those after it (0: none);
 // fake_launches() is the number of launches so far, fake_last_grid() the CTAs of
-// the last one.
+// the last one, fake_live() the cudaMallocAsync allocations not yet freed;
+// fake_capturing(1) has streams report that they are being captured.
 #include <cuda_runtime_api.h>
 
 #include <cstdlib>
 #include <cstring>
 
-static long g_launches = 0, g_fail_at = 0, g_allocs = 0, g_grid = 0;
+static long g_launches = 0, g_fail_at = 0, g_allocs = 0, g_grid = 0, g_live = 0;
+static int g_capturing = 0;
 
 extern "C" {
 
@@ -20,6 +22,8 @@ void fake_fail_allocations(long k) {
 }
 long fake_launches() { return g_launches; }
 long fake_last_grid() { return g_grid; }
+long fake_live() { return g_live; }
+void fake_capturing(int on) { g_capturing = on; }
 
 static cudaError_t give(void **p, size_t n) {
   *p = std::calloc(n ? n : 1, 1);
@@ -33,9 +37,11 @@ static cudaError_t launched(dim3 g) {
 
 cudaError_t cudaMallocAsync(void **p, size_t n, cudaStream_t) {
   if (g_fail_at && ++g_allocs >= g_fail_at) return cudaErrorMemoryAllocation;
+  ++g_live;
   return give(p, n);
 }
 cudaError_t cudaFreeAsync(void *p, cudaStream_t) {
+  --g_live;
   std::free(p);
   return cudaSuccess;
 }
@@ -135,7 +141,7 @@ cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
 cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus *st) {
-  *st = cudaStreamCaptureStatusNone;
+  *st = g_capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
   return cudaSuccess;
 }
 cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaSuccess; }
