@@ -110,15 +110,6 @@ __device__ __noinline__ double2 adi_tbc_rhs(double2 edge, double2 inner, double 
   return cx_div_real_rn(cx_mul_rn(tbc_factor(edge, inner), edge), kd2);
 }
 
-// 1/m for 1e-300 < m < 1e300: the hardware's approximate reciprocal and two
-// Newton steps (error below 2 ulp).  1.0/m adds a branch to a subroutine for
-// other arguments, which the row chain would pay for at every row.
-__device__ __forceinline__ double rcp_newton(double m) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(m));
-  r = fma(r, fma(-m, r, 1.0), r);
-  return fma(r, fma(-m, r, 1.0), r);
-}
 __device__ __forceinline__ double2 crecip_newton(double2 b) {
   const double r = rcp_newton(fma(b.x, b.x, b.y * b.y));
   return mk(b.x * r, -b.y * r);

@@ -71,11 +71,22 @@ __device__ __forceinline__ double2 cx_scale_rn(double2 a, double s) {
 __device__ __forceinline__ double2 cx_div_real_rn(double2 a, double s) {
   return mk(__ddiv_rn(a.x, s), __ddiv_rn(a.y, s));
 }
-// a / s for many a and one s: r = 1/s rounded, then one residual correction of
-// a * r (P. Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", IBM J. Res. Dev. 34(1), 1990): the division's value
-// in three operations instead of a subroutine.  Infinities and NaN pass
-// through as they do in a division.
+// 1/m for a normal m up to 2^1022 by the Newton-Raphson iteration r <- r + r (1 -
+// m r), twice, from the hardware's approximate reciprocal; at most one unit in
+// the last place from the division's value.  1.0/m adds a branch to a subroutine
+// for other arguments, which a chain of rows would pay for at every row.
+__device__ __forceinline__ double rcp_newton(double m) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(m));
+  r = fma(r, fma(-m, r, 1.0), r);
+  return fma(r, fma(-m, r, 1.0), r);
+}
+// a / s for many a and one whole number s: r = 1/s rounded, then one residual
+// correction of a * r (P. Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990): the division's
+// value (a subnormal one to its last place) in three operations instead of a
+// subroutine.  Signed zeros, infinities and NaN pass through as they do in a
+// division.
 struct Divisor {
   double s, r;
 };
@@ -83,7 +94,7 @@ __device__ __forceinline__ Divisor divisor(double s) { return {s, __ddiv_rn(1.0,
 __device__ __forceinline__ double div_by(double a, Divisor d) {
   const double q = __dmul_rn(a, d.r);
   const double c = __fma_rn(__fma_rn(-d.s, q, a), d.r, q);
-  return fabs(q) <= 1.7976931348623157e308 ? c : q;
+  return fabs(q) <= 1.7976931348623157e308 && q != 0.0 ? c : q;
 }
 __device__ __forceinline__ double2 cx_div_by(double2 a, Divisor d) {
   return mk(div_by(a.x, d), div_by(a.y, d));
