@@ -38,8 +38,8 @@ namespace pxp {
 __device__ __forceinline__ void sphere_material(const AdiHalf &h, double x, double y,
                                                 long long idx, double &delta, double &beta) {
   if (h.plane_delta) {
-    delta = h.plane_delta[idx];
-    beta = h.plane_beta[idx];
+    delta = opaque(h.plane_delta[idx]);
+    beta = opaque(h.plane_beta[idx]);
     return;
   }
   if (h.csg.active) {

@@ -89,8 +89,8 @@ int spheres_meeting(const pxp_sphere *spheres, int nspheres, double z, pxp::Sphe
     volatile double r2 = spheres[i].radius * spheres[i].radius;
     if (!(dz2 < r2)) continue;
     if (out && c < pxp::kInlineSpheres)
-      out[c] = {spheres[i].cx, spheres[i].cy, spheres[i].cz, spheres[i].radius, spheres[i].delta,
-                spheres[i].beta};
+      out[c] = {spheres[i].cx, spheres[i].cy, spheres[i].cz, spheres[i].radius,
+                pxp::opaque(spheres[i].delta), pxp::opaque(spheres[i].beta)};
     ++c;
   }
   return c;

@@ -605,6 +605,7 @@ int cn_set_planes(pxp_solver_s *h, const double *delta, const double *beta, int 
     std::memcpy(&buf[2 * per + (size_t)s * n], delta + src1, sizeof(double) * n);
     std::memcpy(&buf[3 * per + (size_t)s * n], beta + src1, sizeof(double) * n);
   }
+  for (double &v : buf) v = pxp::opaque(v);
   h->medium_ok = false;
   h->cn_const = h->cn_vacuum = false;
   cn_win_release(h, h->stream);
@@ -820,7 +821,8 @@ void active_spheres(const pxp_solver_s *h, double z, std::vector<pxp::Sphere> &o
     volatile double dz = z - sp.cz;
     volatile double dz2 = dz * dz;
     volatile double r2 = sp.radius * sp.radius;
-    if (dz2 < r2) out.push_back({sp.cx, sp.cy, sp.cz, sp.radius, sp.delta, sp.beta});
+    if (dz2 < r2)
+      out.push_back({sp.cx, sp.cy, sp.cz, sp.radius, pxp::opaque(sp.delta), pxp::opaque(sp.beta)});
   }
 }
 
@@ -1783,8 +1785,8 @@ int pxp_set_material_spheres(pxp_solver h, const pxp_sphere *spheres, int n) {
   if (n > 0) {
     std::vector<pxp::Sphere> dev(n);
     for (int i = 0; i < n; ++i)
-      dev[i] = {spheres[i].cx, spheres[i].cy, spheres[i].cz, spheres[i].radius, spheres[i].delta,
-                spheres[i].beta};
+      dev[i] = {spheres[i].cx, spheres[i].cy, spheres[i].cz, spheres[i].radius,
+                pxp::opaque(spheres[i].delta), pxp::opaque(spheres[i].beta)};
     int rc;
     if ((rc = alloc(h, (void **)&h->d_spheres, sizeof(pxp::Sphere) * n, "sphere list"))) return rc;
     if (int rc_ = h2d(h, h->d_spheres, dev.data(), sizeof(pxp::Sphere) * n)) return rc_;
@@ -1881,7 +1883,7 @@ int pxp_set_material_csg(pxp_solver h, const pxp_csg_module *modules, int nmodul
   pxp::CsgShape *ds = (pxp::CsgShape *)(dp + nparts);
   for (int m = 0; m < nmodules; ++m) dm[m] = {modules[m].first_part, modules[m].num_parts};
   for (int p = 0; p < nparts; ++p)
-    dp[p] = {parts[p].delta, parts[p].beta, parts[p].operation, parts[p].first_shape, parts[p].num_shapes};
+    dp[p] = {pxp::opaque(parts[p].delta), pxp::opaque(parts[p].beta), parts[p].operation, parts[p].first_shape, parts[p].num_shapes};
   for (int k = 0; k < nshapes; ++k) {
     pxp::CsgShape c{};
     for (int j = 0; j < 12; ++j) c.m[j] = shapes[k].transform[j];
