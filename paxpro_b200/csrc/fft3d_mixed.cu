@@ -6,7 +6,7 @@
 // The same two passes per step as fft3d.cu (x pass: F_x, K, F_x^-1; y pass:
 // F_y^-1, refraction, F_y), each line transform mixed-radix (fft_mixed.cuh).
 // A CTA holds L adjacent lines, TL threads each, in two buffers a line; the
-// line's threads synchronise among themselves only (a warp, or a named
+// line's threads synchronise among themselves only (a named
 // barrier), so lines drift apart and one's loads cover another's arithmetic.
 // Lines come and go cooperatively: contiguous lines as whole runs, strided
 // ones as L adjacent elements a position.
@@ -43,10 +43,7 @@ __global__ void __launch_bounds__(TL *L) fft3d_mixed_kernel(const __grid_constan
   const int nl = n - line0 < L ? n - line0 : L;  // lines of this CTA
   C *field = reinterpret_cast<C *>(q.field);
   const bool strided = q.mode == 1;  // x lines: fixed row, stride n
-  auto sync = [slot] {
-    if constexpr (TL == 32) __syncwarp();
-    else asm volatile("bar.sync %0, %1;\n" ::"r"(1 + slot), "n"(TL) : "memory");
-  };
+  auto sync = [slot] { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + slot), "n"(TL) : "memory"); };
 
   // the table does not depend on the previous kernel: copied while it drains
   for (int i = tid; i < plan.table; i += T)
@@ -119,7 +116,7 @@ __global__ void __launch_bounds__(TL *L) fft3d_mixed_kernel(const __grid_constan
 
 template <typename R, int TL, int L, bool BIG>
 cudaError_t launch_t(const Fft3dPass &q, const MixedPlan &plan, const double *kx2, cudaStream_t s) {
-  const size_t smem = 2 * sizeof(typename Cx<R>::T) * L * plan.n + 16 * (size_t)plan.table;
+  const size_t smem = mixed_lines_smem(plan, L, sizeof(R) == 4);
   if (smem > 227 * 1024) return cudaErrorInvalidValue;
   auto k = fft3d_mixed_kernel<R, TL, L, BIG>;
   const cudaError_t e = raise_dynamic_smem((const void *)k, (int)smem);
@@ -147,16 +144,10 @@ cudaError_t launch_b(const Fft3dPass &q, const MixedPlan &plan, const double *kx
 
 template <typename R>
 cudaError_t launch_r(const Fft3dPass &q, const MixedPlan &plan, const double *kx2, cudaStream_t s) {
-  // lines a CTA and threads a line: short lines one a CTA (300 nodes: 14.8 us a
-  // step against 17.8 with two of 64 threads); around 513 nodes, whose primes
-  // give a pass few butterflies, 64 threads (29 us; 128: 39); above, complex64
-  // lines keep 64 threads (1000: 49 us; 128: 57), complex128 lines take 128
-  // (61 us; 64: 73)
-  const int n = plan.n;
-  if (n <= 400) return launch_b<R, 128, 1>(q, plan, kx2, s);
-  if (n <= (sizeof(R) == 4 ? 1200 : 700)) return launch_b<R, 64, 2>(q, plan, kx2, s);
-  if (n <= 2700) return launch_b<R, 128, 2>(q, plan, kx2, s);
-  return launch_b<R, 256, 1>(q, plan, kx2, s);
+  const MixedLines l = mixed_lines(plan.n, sizeof(R) == 4);
+  if (l.lines == 2)
+    return l.threads == 64 ? launch_b<R, 64, 2>(q, plan, kx2, s) : launch_b<R, 128, 2>(q, plan, kx2, s);
+  return l.threads == 128 ? launch_b<R, 128, 1>(q, plan, kx2, s) : launch_b<R, 256, 1>(q, plan, kx2, s);
 }
 
 }  // namespace
