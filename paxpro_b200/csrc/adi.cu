@@ -1041,17 +1041,14 @@ static cudaError_t adi_const_wave_launch(const AdiHalf &h, const void *tabs, cud
                            : adi_const_wave_launch_x<R, N, M, G, S, false>(h, tabs, s);
 }
 
-// (M, G) of the one-wave kernel per size: each system group holds whole
-// warps (n/M a multiple of 32) and ceil(n / G) CTAs fill the SMs about once.
-static bool adi_wave_config(int n, int *m, int *g) {
+// Rows a thread of the one-wave kernel for a system length adi_wave_n gives
+// (whole warps a system: n / M a multiple of 32), 0 for others.
+static int adi_wave_rows(int n) {
   switch (n) {
-    case 64: *m = 2; *g = 4; return true;
-    case 128: *m = 4; *g = 2; return true;
-    case 256: *m = 8; *g = 2; return true;
-    case 512: *m = 8; *g = 4; return true;
-    case 768: *m = 8; *g = 6; return true;
-    case 1024: *m = 8; *g = 7; return true;
-    default: return false;
+    case 64: return 2;
+    case 128: return 4;
+    case 256: case 512: case 768: case 1024: return 8;
+    default: return 0;
   }
 }
 
@@ -1064,8 +1061,8 @@ int adi_wave_n(int n) {
 }
 
 bool adi_const_staged_tables(int n, const double *g, const double *h, double *out, int run[2]) {
-  int M = 0, G = 0;
-  if (!adi_wave_config(n, &M, &G)) return false;
+  const int M = adi_wave_rows(n);
+  if (M == 0) return false;
   const int P = n / M;
   auto slot = [&](int c, int m) { return m * P + (c ^ (m & 7)); };
   // the device's cmul: (fma(ax, bx, -ay*by), fma(ax, by, ay*bx))

@@ -43,8 +43,6 @@ void set_global_error(const std::string &m) {
   g_last_error = m;
 }
 
-bool is_pow2(long long n) { return n > 0 && (n & (n - 1)) == 0; }
-
 }  // namespace
 
 void pxp::set_last_error(const char *msg) { set_global_error(msg ? msg : ""); }
@@ -222,21 +220,6 @@ cd transmission(double k, double beta, double delta, double dz) {
 int h2d(pxp_solver_s *h, void *dst, const void *src, size_t bytes) {
   PXP_TRY_CUDA(h, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->stream));
   PXP_TRY_CUDA(h, cudaStreamSynchronize(h->stream));
-  return PXP_OK;
-}
-
-// Upload complex128 host values in the solver's precision.
-int upload_complex(pxp_solver_s *h, void *dst, const cd *src, long long n) {
-  if (h->prec == pxp::kFP64) {
-    if (int rc_ = h2d(h, dst, src, sizeof(cd) * n)) return rc_;
-  } else {
-    std::vector<float> tmp(2 * n);
-    for (long long i = 0; i < n; ++i) {
-      tmp[2 * i] = (float)src[i].real();
-      tmp[2 * i + 1] = (float)src[i].imag();
-    }
-    if (int rc_ = h2d(h, dst, tmp.data(), sizeof(float) * 2 * n)) return rc_;
-  }
   return PXP_OK;
 }
 

@@ -37,11 +37,8 @@ namespace cg = cooperative_groups;
 
 namespace pxp {
 
-// Coefficients of row i (exact FP64, reference operation order).
-struct CnRow {
-  double2 diag, rhs;
-};
-
+// Diagonal of row i and its right-hand side (exact FP64, reference operation
+// order).
 __device__ __forceinline__ double2 cn_diag(double delta, double beta, double rho, double r) {
   // fval*1.0 + 0.25*(H+ + H-)*g*i*rho + 0.5*(beta*r + i*delta*r)
   double im_a = __dmul_rn(0.5, rho);              // 0.25*(1+1)*1 = 0.5, *i, *rho

@@ -104,6 +104,7 @@ template <typename R, int N, int LG> struct Cfg {
   // addresses, known at compile time with two copies, count (4096: 483 -> 510
   // with one, 256: 7.6 -> 7.8).
   static constexpr bool ONE_DIR = sizeof(R) == 4;
+  static_assert(!(ONE_DIR && WARP_ST), "the warps' stores do not swap");
   static_assert(N % 8 == 0 && T <= 1024, "line slots");
 };
 
@@ -431,7 +432,7 @@ __global__ void __launch_bounds__(Cfg<R, N, LG>::T, Cfg<R, N, LG>::MINB)
       const int lane = tid & 31, w0 = tid & ~31;
       __syncwarp();
 #pragma unroll
-      for (int s = 0; s < 8; ++s) F[j + s * K::TL] = K::ONE_DIR ? swapri(v[0][s]) : v[0][s];
+      for (int s = 0; s < 8; ++s) F[j + s * K::TL] = v[0][s];
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       __syncwarp();
       if (lane == 0) {
