@@ -527,10 +527,8 @@ __device__ __forceinline__ void pivot_sum(double b, QSq q2, double hi, double lo
   const double bb = __dsub_rn(s, b);
   t = __dadd_rn(__dadd_rn(__dsub_rn(b, __dsub_rn(s, bb)), __dsub_rn(p, bb)), e);
 }
-__device__ __forceinline__ PivotInv pivot_inverse(double2 b, QSq q2, PivotInv prev) {
-  double2 d, dl;
-  pivot_sum(b.x, q2, prev.hi.x, prev.lo.x, d.x, dl.x);
-  pivot_sum(b.y, q2, prev.hi.y, prev.lo.y, d.y, dl.y);
+// 1 / (d + dl), dl the second word of d.
+__device__ __forceinline__ PivotInv inverse_words(double2 d, double2 dl) {
   const double2 r = crecip(d);
   // residual 1 - (d + dl) r
   const double p1 = __dmul_rn(d.x, r.x), p2 = __dmul_rn(d.y, r.y);
@@ -544,6 +542,34 @@ __device__ __forceinline__ PivotInv pivot_inverse(double2 b, QSq q2, PivotInv pr
   const double ry = -(p3 + p4) - (__fma_rn(d.x, r.y, -p3) + __fma_rn(d.y, r.x, -p4)) -
                     (dl.x * r.y + dl.y * r.x);
   return {r, cmul(r, mk(rx, ry))};
+}
+__device__ __forceinline__ PivotInv pivot_inverse(double2 b, QSq q2, PivotInv prev) {
+  double2 d, dl;
+  pivot_sum(b.x, q2, prev.hi.x, prev.lo.x, d.x, dl.x);
+  pivot_sum(b.y, q2, prev.hi.y, prev.lo.y, d.y, dl.y);
+  return inverse_words(d, dl);
+}
+
+// hi + lo rounded to one word, up or down by a draw of 32 bits with probabilities
+// that make the mean exact (G. E. Forsythe, "Round-off errors in numerical
+// integration on automatic machinery", Bull. AMS 56, 1950).  Rounded to
+// nearest, a table entry errs the same way at every row of a uniform stretch and
+// at every step, and the errors of a pass add up; this way they do not.
+__device__ __forceinline__ double round_dithered(double hi, double lo, unsigned draw) {
+  const double s = __dadd_rn(hi, lo), t = __dsub_rn(lo, __dsub_rn(s, hi));
+  const double top = __longlong_as_double(__double_as_longlong(s) & 0x7ff0000000000000ll);
+  // the draw, -1/2 .. 1/2 units in the last place of s
+  return __dadd_rn(s, __fma_rn((double)(int)draw * 5.1698788284564230e-26, top, t));
+}
+// A draw for entry k of a step: the finalizer of MurmurHash3 (A. Appleby, public
+// domain) over both.
+__device__ __forceinline__ unsigned dither(unsigned step, unsigned k) {
+  unsigned h = step * 0x9e3779b1u + k;
+  h ^= h >> 16;
+  h *= 0x85ebca6bu;
+  h ^= h >> 13;
+  h *= 0xc2b2ae35u;
+  return h ^ (h >> 16);
 }
 
 // Pivots of one recurrence of a step: row k (from the left, or DIR < 0 from the
@@ -648,14 +674,20 @@ __global__ void __launch_bounds__(TT)
   QSq q2;
   q2.hi = __dmul_rn(q, q);
   q2.lo = __fma_rn(q, q, -q2.hi);
+  auto draw = [step = pw.first + st](int row, int k) { return dither((unsigned)step, (unsigned)row * 8u + k); };
   double2 *out = pw.tabs + st * cn_step_entries(M, TT);
   double2 aL = mk(1.0, 0.0), aR = mk(1.0, 0.0);
 #pragma unroll
   for (int m = 0; m < M; ++m) {
     const int i = t * M + m;
     const PivotInv il = pivot(0, i - 1), ir = pivot(1, i + 1);
-    const double2 hL = mk(-fma(q, il.hi.y, q * il.lo.y), fma(q, il.hi.x, q * il.lo.x));
-    const double2 hR = mk(-fma(q, ir.hi.y, q * ir.lo.y), fma(q, ir.hi.x, q * ir.lo.x));
+    // i q / pivot
+    auto off = [q](double hi, double lo, unsigned d) {
+      const double p = __dmul_rn(q, hi);
+      return round_dithered(p, __fma_rn(q, lo, __fma_rn(q, hi, -p)), d);
+    };
+    const double2 hL = mk(-off(il.hi.y, il.lo.y, draw(i, 0)), off(il.hi.x, il.lo.x, draw(i, 1)));
+    const double2 hR = mk(-off(ir.hi.y, ir.lo.y, draw(i, 2)), off(ir.hi.x, ir.lo.x, draw(i, 3)));
     double2 c = mk(2.0, 0.0), b = mk(kCnPad, 0.0);
     if (i < n) {
       b = cn_diag(de[i], be[i], job.rho, job.r);
@@ -667,7 +699,9 @@ __global__ void __launch_bounds__(TT)
     pivot_sum(b.y, q2, il.hi.y, il.lo.y, d.y, dl.y);
     pivot_sum(d.x, q2, ir.hi.x, ir.lo.x, f.x, fl.x);
     pivot_sum(d.y, q2, ir.hi.y, ir.lo.y, f.y, fl.y);
-    const double2 w = crecip(mk(f.x + (fl.x + dl.x), f.y + (fl.y + dl.y)));
+    const PivotInv wi = inverse_words(f, mk(fl.x + dl.x, fl.y + dl.y));
+    const double2 w = mk(round_dithered(wi.hi.x, wi.lo.x, draw(i, 4)),
+                         round_dithered(wi.hi.y, wi.lo.y, draw(i, 5)));
     out[m * TT + t] = c;
     out[(M + m) * TT + t] = hL;
     out[(2 * M + m) * TT + t] = hR;
@@ -718,9 +752,11 @@ constexpr bool cn_c_in_registers(int M, int T) { return M * T > 1024; }
 // cn_kernel): 300 rows 1.0 and 75 (8.2), 1000: 1.2 and 157 (10.8), 1501: 1.9 and
 // 218 (15.1), 4000: 1.9 and 513 (27); eight problems of 1501 rows and 200 steps
 // in a batch 0.91 ms (3.17), 40 of them 2.1 (3.7), 148, whose 11 GB of pivots
-// and tables go through HBM, 9.7 (5.6).  Errors against an 80-bit sweep, 1501
-// and 3000 rows: 0.05 .. 0.2e-12 and 0.04 .. 0.6e-12 (step by step 2e-13 and
-// 2e-12; with pivots of one word 1.4e-12 and 2.2e-12).
+// and tables go through HBM, 9.7 (5.6).  Errors against an 80-bit sweep after
+// 300 steps, the median of three guides (step by step; with entries rounded to
+// nearest): 64 rows 4e-15 (6e-15; 4e-14), 128: 3e-15 (9e-15; 2e-14), 300: 3e-15
+// (6e-15; 2e-14), 1000: 1.4e-14 (3e-14; 5e-14), 3000: 2e-14 (2e-12; 9e-14); with
+// pivots of one word 1501 and 3000 rows 1.4e-12 and 2.2e-12.
 template <typename R, int M, int T, int K, bool FLUX>
 __global__ void __launch_bounds__(T) cn_planes_kernel(const CnJob *__restrict__ jobs,
                                                      const CnPlanes *__restrict__ list,
