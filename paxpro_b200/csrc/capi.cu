@@ -114,7 +114,7 @@ struct pxp_solver_s {
   // false from the moment a material call starts to replace the medium until it
   // has done so: after a failed one the old tables and planes are gone
   bool medium_ok = true;
-  bool counted = false;  // among handle_count
+  bool busy = false;  // work enqueued that the host has not waited for: among busy_handles
   bool ic_set = false;
   unsigned current_step = 1;
   // the device's count of ran-out kernel waits (wait_counter.cu): the host's
@@ -1250,21 +1250,25 @@ cudaError_t cn_planes_steps(pxp_solver_s *h, long long first, int nsteps, int ot
   return e;
 }
 
-// Handles of the process per device and dimension.  They may be stepping on
-// streams of their own beside a launch, which takes its size from them
-// (launch_cn_const); results never depend on it.
+// Handles of the process per device and dimension that have been given work
+// (initial conditions or steps) since the host last waited for them.  They may be
+// stepping on streams of their own beside a launch, which takes its size from
+// them (launch_cn_const); results never depend on it.
 constexpr int kMaxDevices = 64;  // as wait_counter
-std::atomic<int> g_handles_2d[kMaxDevices], g_handles_3d[kMaxDevices];
+std::atomic<int> g_busy_2d[kMaxDevices], g_busy_3d[kMaxDevices];
 
-std::atomic<int> &handle_count(const pxp_solver_s *h) {
+void set_busy(pxp_solver_s *h, bool busy) {
+  if (h->busy == busy) return;
+  h->busy = busy;
   const bool d2 = h->prob.kind == PXP_FFT_SOLVER_2D || h->prob.kind == PXP_CRANK_NICHOLSON;
-  return (d2 ? g_handles_2d : g_handles_3d)[h->prob.device];
+  (d2 ? g_busy_2d : g_busy_3d)[h->prob.device] += busy ? 1 : -1;
 }
 
-// SMs that the device's handles other than the nj of a launch may be using.
+// SMs that the device's handles other than the nj of a launch (busy themselves)
+// may be using.
 int sms_of_others(int device, int nj) {
   constexpr int kAll = 1 << 20;
-  return g_handles_3d[device] > 0 ? kAll : std::max(0, g_handles_2d[device] - nj);
+  return g_busy_3d[device] > 0 ? kAll : std::max(0, g_busy_2d[device] - nj);
 }
 
 int cn_write_job(pxp_solver_s *h);
@@ -1602,15 +1606,13 @@ int pxp_solver_create(const pxp_problem *problem, pxp_solver *out) {
       break;
   }
   h->medium_ok = true;
-  ++handle_count(h);
-  h->counted = true;
   *out = h;
   return PXP_OK;
 }
 
 int pxp_solver_destroy(pxp_solver h) {
   if (h == nullptr) return PXP_OK;
-  if (h->counted) --handle_count(h);
+  set_busy(h, false);
   if (h->stream) cudaStreamSynchronize(h->stream);
   if (h->graph) cudaGraphExecDestroy(h->graph);
   h->graph = nullptr;
@@ -1914,6 +1916,7 @@ static int waits_held(pxp_solver_s *h) {
 }
 static int check_waits(pxp_solver_s *h) {
   PXP_TRY_CUDA(h, cudaStreamSynchronize(h->stream));
+  set_busy(h, false);
   return waits_held(h);
 }
 
@@ -1937,6 +1940,7 @@ int pxp_set_initial_conditions(pxp_solver h, const double *field) {
   h->current_step = 1;
   h->cn_win_count = 0;  // tables serve one pass through the medium
   h->ic_set = true;
+  set_busy(h, true);
   return PXP_OK;
 }
 
@@ -1947,6 +1951,7 @@ int pxp_set_initial_conditions_device(pxp_solver h, const void *dfield) {
   h->current_step = 1;
   h->cn_win_count = 0;
   h->ic_set = true;
+  set_busy(h, true);
   return PXP_OK;
 }
 
@@ -1963,6 +1968,7 @@ int pxp_step(pxp_solver h, int nsteps) {
       (first < h->plane_first || last >= (long long)h->plane_first + h->plane_count))
     return h->fail(PXP_ERR_INVALID, "steps " + std::to_string(first) + ".." + std::to_string(last) +
                                         " are outside the material planes provided");
+  set_busy(h, true);
   cudaError_t e = cudaSuccess;
   switch (h->prob.kind) {
     case PXP_FFT_SOLVER_2D:
@@ -2700,8 +2706,10 @@ int pxp_batch_round(pxp_batch b, int max_steps) {
   if (b == nullptr || max_steps <= 0) return PXP_ERR_INVALID;
   cudaSetDevice(b->device);
   for (pxp_solver_s *h : b->active)
-    if (h->batch_remaining > 0)
+    if (h->batch_remaining > 0) {
       if (int rc = check_medium(h)) return b->fail(rc, h->err);
+      set_busy(h, true);
+    }
   // the staging buffer of the previous round must be consumed
   if (cudaStreamSynchronize(b->stream) != cudaSuccess) return b->fail(PXP_ERR_CUDA, "batch stream");
   // ---- 2-D groups: key (kind, n, precision, CN path: 0 step by step, 1 a
@@ -2892,6 +2900,7 @@ int pxp_batch_collect(pxp_batch b, pxp_solver *done, int cap, int *count) {
   for (pxp_solver_s *h : b->active) {
     if (!is_2d(h) && cudaStreamSynchronize(h->stream) != cudaSuccess)
       return b->fail(PXP_ERR_CUDA, "solver stream");
+    set_busy(h, false);
     if (h->batch_remaining <= 0 && c < cap) {
       done[c++] = h;
       b->used -= h->dev_bytes;

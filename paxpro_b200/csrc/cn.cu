@@ -914,8 +914,8 @@ bool cn_const_supported(Precision, int n) {
 // two, 1.42 on four; 8192 in FP32: 2.93 on two, 2.09 on four; 16384: 2.79 on
 // four, 2.07 on eight), at more SM time a problem.  The widest form runs for
 // which every problem of the launch finds its SMs free beside the `others` that
-// the caller's other handles may be using: an SM for each handle of a 2-D kind,
-// all of them for one of a 3-D kind.  (A 1024^2 ADI half step is one wave of 147
+// the caller's other handles with work enqueued may be using: an SM for each of a
+// 2-D kind, all of them for one of a 3-D kind.  (A 1024^2 ADI half step is one wave of 147
 // CTAs, an SM each: beside a problem on four SMs it takes two waves, 40 us a
 // step against 22.9.)  The forms have the same chunks and warps and give the
 // same bits.  2048 rows gain too little (1.40 on one SM, 1.31 on two).

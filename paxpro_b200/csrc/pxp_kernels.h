@@ -134,7 +134,7 @@ constexpr double kCnPad = 1e30;
 // z-invariant medium and Dirichlet ends: the step matrix never changes; the
 // job's lu_l / lu_r / lu_w hold hL, hR and 2 w of the two-sided solve (n
 // complex128 each, see cn.cu).  others: SMs that other handles of the device
-// may be using.
+// with work enqueued may be using.
 cudaError_t launch_cn_const(Precision p, const CnJob *d_jobs, int nj, int n, int step0,
                             int nsteps, cudaStream_t s, bool flux, int others);
 bool cn_const_supported(Precision p, int n);

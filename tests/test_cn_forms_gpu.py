@@ -29,6 +29,7 @@ def test_forms_agree(n, precision):
     assert len(alone) == 5 and np.all(np.isfinite(alone[0]))
     x = pxp.Disc(-500.0, 500.0, wl.step_for_nodes(-500.0, 500.0, 16))
     third = pxp.Solver(pxp.ProblemSpec(kind=pxp.ADI, x=x, y=x, z=pxp.Disc(0.0, 1e4, 1000.0), wavenumber=wl.K))
+    third.set_initial_conditions(np.ones((16, 16), dtype=np.complex128))  # at work until waited for
     with result(_solver(pxp, n, nsteps, precision, 8)) as s:
         s.step(nsteps)
         beside = read(s)

@@ -75,6 +75,7 @@ def test_splits_and_batches_give_the_same_bits(n, nsteps, precision):
     started.step(2)
     x = pxp.Disc(-500.0, 500.0, wl.step_for_nodes(-500.0, 500.0, 16))
     third = pxp.Solver(pxp.ProblemSpec(kind=pxp.ADI, x=x, y=x, z=pxp.Disc(0.0, 1e4, 1000.0), wavenumber=wl.K))
+    third.set_initial_conditions(np.ones((16, 16), dtype=np.complex128))  # at work until waited for
     batch = pxp.Batch()
     for i, (s, _) in enumerate(jobs):
         assert batch.admit(s, nsteps - 3 * i if nsteps > 20 else nsteps)
