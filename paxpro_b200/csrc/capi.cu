@@ -1160,11 +1160,13 @@ size_t cn_win_step_bytes(const pxp_solver_s *h) {
   return pxp::cn_table_bytes(n) + pxp::cn_pivot_bytes(n);
 }
 
-// Steps of a buffer of at most `bytes`, for windows from `step` on.
+// Steps of a buffer of at most `bytes`, for windows from `step` on (whole warps of
+// the pivot kernel).
 int cn_win_steps(const pxp_solver_s *h, long long step, size_t bytes) {
-  const size_t per = cn_win_step_bytes(h);
   const long long left = (long long)h->plane_first + h->plane_count - step;
-  return (int)std::min<long long>(left, std::max<long long>(1, (long long)(bytes / per)));
+  long long fit = std::max<long long>(1, (long long)(bytes / cn_win_step_bytes(h)));
+  if (fit > 32) fit -= fit % 32;
+  return (int)std::min(left, fit);
 }
 
 // Whether the handle has a buffer for the tables of `step` and the steps after it
@@ -2586,8 +2588,10 @@ bool cn_uses_const(const pxp_solver_s *h) {
   return h->cn_const && !h->prob.transparent_bc && h->mat_stride == 0;
 }
 
-// A batch's windows of sampled media, all jobs together.
-constexpr size_t kCnBatchBytes = size_t(12) << 30;
+// A batch's windows of sampled media, all jobs together.  (The pool grows by some 12
+// us a MB the first time, and keeps it; 8, 40 and 80 jobs of 1501 rows and 200
+// steps take 0.75, 1.6 and 2.9 ms with 2 GB, 0.75, 1.5 and 2.9 with 12.)
+constexpr size_t kCnBatchBytes = size_t(2) << 30;
 
 // A launch of a group of sampled-media jobs: every job's part of it.
 struct CnPart {
@@ -2713,7 +2717,8 @@ int pxp_batch_round(pxp_batch b, int max_steps) {
   // the staging buffer of the previous round must be consumed
   if (cudaStreamSynchronize(b->stream) != cudaSuccess) return b->fail(PXP_ERR_CUDA, "batch stream");
   // ---- 2-D groups: key (kind, n, precision, CN path: 0 step by step, 1 a
-  // step-invariant matrix, 2 tables of sampled media, the paths of pxp_step)
+  // step-invariant matrix, 2 tables of sampled media: the paths of pxp_step, but
+  // for large groups of sampled media, which go step by step)
   struct Key {
     int kind, n, prec, cpath;
     bool operator<(const Key &o) const {
@@ -2721,16 +2726,24 @@ int pxp_batch_round(pxp_batch b, int max_steps) {
     }
   };
   std::map<Key, std::vector<pxp_solver_s *>> groups;
-  size_t sampled = 0;
-  for (const pxp_solver_s *h : b->active) sampled += h->batch_remaining > 0 && cn_uses_planes(h);
+  auto key = [](const pxp_solver_s *h, int cpath) {
+    return Key{h->prob.kind, (int)h->nx, (int)h->prec, cpath};
+  };
+  std::map<Key, int> sampled;  // the jobs of each size whose media have tables when alone
+  for (const pxp_solver_s *h : b->active)
+    if (h->batch_remaining > 0 && cn_uses_planes(h)) ++sampled[key(h, 2)];
+  auto with_tables = [&](const pxp_solver_s *h) {
+    return cn_uses_planes(h) && pxp::cn_planes_pay(pxp::cn_padded_n((int)h->nx), sampled[key(h, 2)]);
+  };
+  size_t windows = 0;
+  for (const pxp_solver_s *h : b->active) windows += h->batch_remaining > 0 && with_tables(h);
   for (pxp_solver_s *h : b->active) {
     if (!is_2d(h) || h->batch_remaining <= 0) continue;
-    Key k{h->prob.kind, (int)h->nx, (int)h->prec, 0};
-    if (h->prob.kind == PXP_CRANK_NICHOLSON && cn_uses_const(h)) k.cpath = 1;
-    if (cn_uses_planes(h) &&
-        cn_win_reserve(h, h->current_step, std::min(kCnWindowBytes, kCnBatchBytes / sampled), b->stream))
-      k.cpath = 2;
-    groups[k].push_back(h);
+    int cpath = h->prob.kind == PXP_CRANK_NICHOLSON && cn_uses_const(h) ? 1 : 0;
+    if (with_tables(h) &&
+        cn_win_reserve(h, h->current_step, std::min(kCnWindowBytes, kCnBatchBytes / windows), b->stream))
+      cpath = 2;
+    groups[key(h, cpath)].push_back(h);
   }
   // Within a group the CTA index follows the job order, and the block
   // scheduler starts CTAs in index order as SMs free up: with the jobs that
@@ -2867,9 +2880,14 @@ int pxp_batch_round(pxp_batch b, int max_steps) {
           if (next >= (long long)h->cn_win_first + h->cn_win_count) cn_win_release(h, gst);
         }
     }
-    else
+    else {
       e = pxp::launch_cn((pxp::Precision)k.prec, (const pxp::CnJob *)jobs, (int)list.size(),
                          pxp::cn_padded_n(k.n), -1, -1, gst, any_flux);
+      for (pxp_solver_s *h : list) {  // a window from steps taken otherwise
+        const long long next = (long long)h->current_step + std::min(h->batch_remaining, max_steps);
+        if (next >= (long long)h->cn_win_first + h->cn_win_count) cn_win_release(h, gst);
+      }
+    }
     if (e != cudaSuccess) return b->fail(PXP_ERR_CUDA, std::string("batch launch: ") + cudaGetErrorString(e));
     if (cudaEventRecord(b->gdone[gi], gst) != cudaSuccess ||
         cudaStreamWaitEvent(b->stream, b->gdone[gi], 0) != cudaSuccess)

@@ -751,8 +751,7 @@ constexpr bool cn_c_in_registers(int M, int T) { return M * T > 1024; }
 // window.  Measured, us a step and us of pivots a window (step by step,
 // cn_kernel): 300 rows 1.0 and 75 (8.2), 1000: 1.2 and 157 (10.8), 1501: 1.9 and
 // 218 (15.1), 4000: 1.9 and 513 (27); eight problems of 1501 rows and 200 steps
-// in a batch 0.91 ms (3.17), 40 of them 2.1 (3.7), 148, whose 11 GB of pivots
-// and tables go through HBM, 9.7 (5.6).  Errors against an 80-bit sweep after
+// in a batch 0.75 ms (3.1), 48 of them 1.8 (3.1).  Errors against an 80-bit sweep after
 // 300 steps, the median of three guides (step by step; with entries rounded to
 // nearest): 64 rows 4e-15 (6e-15; 4e-14), 128: 3e-15 (9e-15; 2e-14), 300: 3e-15
 // (6e-15; 2e-14), 1000: 1.4e-14 (3e-14; 5e-14), 3000: 2e-14 (2e-12; 9e-14); with
@@ -974,6 +973,18 @@ static cudaError_t cn_planes_launch_t(const CnJob *d_jobs, const CnPlanes *d_lis
 // here: 100 rows 98, 137 and 56, 64; 300: 150, 215 and 90, 98; 1000: 194, 280 and
 // 177, 186; 1501: 262, 383 and 249, 264; 4000: 456, 672 and 545, 559).
 bool cn_planes_supported(int n, int planes) { return n >= 64 && n <= 4096 && planes >= 24; }
+
+// The tables spread a problem's work over SMs that a single one leaves idle; many
+// problems side by side fill the SMs anyway, and theirs go through HBM (280 bytes a
+// row and step).  Measured with 200 steps in a batch, ms step by step and with
+// tables: 250 rows, 148 problems 1.34 and 1.28; 500 rows, 96: 1.83 and 1.40, 148:
+// 1.85 and 2.20; 1000 rows, 96: 2.30 and 2.12, 148: 2.33 and 3.30; 1501 rows, 80:
+// 3.13 and 2.90, 96: 3.13 and 3.26, 148: 3.16 and 5.03; 2048 rows, 64: 3.30 and
+// 2.84, 80: 3.32 and 3.63; 4000 rows, 48: 5.50 and 4.95, 64: 5.51 and 6.89, 148:
+// 5.54 and 11.8.
+bool cn_planes_pay(int n, int nj) {
+  return nj <= (n <= 256 ? 148 : n <= 512 ? 120 : n <= 1024 ? 100 : n <= 2048 ? 72 : 48);
+}
 
 // Chunk and threads of a problem of n padded rows (64 .. 4096).
 static void cn_planes_shape(int n, int *m, int *tt) {

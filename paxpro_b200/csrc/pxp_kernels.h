@@ -150,6 +150,9 @@ struct CnPlanes {
   int step0, nsteps;  // the steps to solve, inside the window (may be none)
 };
 bool cn_planes_supported(int n, int planes);
+// Whether nj such problems side by side are faster that way than step by step
+// (launch_cn).
+bool cn_planes_pay(int n, int nj);
 size_t cn_table_bytes(int n);
 size_t cn_pivot_bytes(int n);
 // nj problems, each with its job and its entry of d_list (null: one problem,

@@ -118,3 +118,29 @@ def test_media_of_few_and_many_steps_in_one_batch():
         s.close()
     const.close()
     batch.close()
+
+
+@pytest.mark.parametrize("n,count,precision,tol", [(300, 121, 0, 1e-12), (1501, 73, 0, 1e-12), (4000, 49, 1, 1e-5)])
+def test_large_groups_agree_with_alone(n, count, precision, tol):
+    """One job more than take the tables: step by step, then the rest with them."""
+    import paxpro_b200 as pxp
+    jobs = [_solver(n, 30, precision, seed=i % 3) for i in range(count)]
+    jobs[0].step(4)
+    batch = pxp.Batch()
+    for i, s in enumerate(jobs):
+        assert batch.admit(s, 26 if i == 0 else 30 if i % 8 else 12)
+    for k in (5, 7, 30):
+        batch.round(k)
+    assert len(batch.collect()) == count
+    alone = []
+    for i in range(3):
+        with _solver(n, 30, precision, seed=i) as s:
+            s.step(12)
+            alone.append([s.get_last_solution()])
+            s.step(18)
+            alone[-1].append(s.get_last_solution())
+    for i, s in enumerate(jobs):
+        want, got = alone[i % 3][1 if i == 0 or i % 8 else 0], s.get_last_solution()
+        assert np.linalg.norm(got - want) <= tol * np.linalg.norm(want)
+        s.close()
+    batch.close()

@@ -105,3 +105,34 @@ def test_captured_steps_bring_their_own_window():
         assert launches(s.step, 5) == 1
         assert launches(s.step, 40) == 1 and fake.fake_live() == held
     """)
+
+
+def test_large_batches_go_step_by_step():
+    fake_cuda.run("""
+        def solver(n, steps):
+            s = pxp.Solver(spec(pxp.CRANK_NICHOLSON, n))
+            z = np.zeros((2 * steps, n))
+            s.set_material_planes(z, z, 1, steps)
+            s.set_initial_conditions(np.ones(n, dtype=np.complex128))
+            return s
+
+        def launches(f, *a):
+            before = fake.fake_launches()
+            f(*a)
+            return fake.fake_launches() - before
+
+        for n, most in ((250, 148), (500, 120), (1000, 100), (2048, 72), (2049, 48)):
+            b = pxp.Batch()
+            jobs = [solver(n, 26) for _ in range(most + 1)]
+            jobs[0].step(2)
+            for i, j in enumerate(jobs):
+                assert b.admit(j, 6 if i in (0, most) else 16)
+            assert launches(b.round, 5) == 1, n
+            assert launches(b.round, 1) == 1 and len(b.collect()) == 2
+            assert launches(b.round, 6) == 3, n  # most - 1 of them
+            assert b.admit(jobs[0], 4)
+            assert launches(b.round, 2) == 1, n  # its window is from its first steps
+            for j in jobs:
+                j.close()
+            b.close()
+    """)
