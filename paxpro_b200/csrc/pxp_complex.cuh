@@ -93,8 +93,9 @@ struct Divisor {
 __device__ __forceinline__ Divisor divisor(double s) { return {s, __ddiv_rn(1.0, s)}; }
 __device__ __forceinline__ double div_by(double a, Divisor d) {
   const double q = __dmul_rn(a, d.r);
-  const double c = __fma_rn(__fma_rn(-d.s, q, a), d.r, q);
-  return fabs(q) <= 1.7976931348623157e308 && q != 0.0 ? c : q;
+  // the negated residual: the corrected quotient of a zero keeps its sign
+  const double c = __fma_rn(-__fma_rn(d.s, q, -a), d.r, q);
+  return fabs(q) <= 1.7976931348623157e308 ? c : q;
 }
 __device__ __forceinline__ double2 cx_div_by(double2 a, Divisor d) {
   return mk(div_by(a.x, d), div_by(a.y, d));
