@@ -504,8 +504,9 @@ static cudaError_t adi_const_launch(const AdiHalf &h, const void *g, const void 
   return cudaGetLastError();
 }
 
-// Vacuum half step, FP64, n <= 1024, one wave: G systems per CTA so that
-// ceil(n / G) CTAs cover the 148 SMs once (G = 7 at n = 1024: 147 CTAs).
+// Vacuum half step, n <= 1024, one wave: G systems per CTA so that ceil(n / G)
+// CTAs fit the 148 SMs at once (G = 7 at n = 1024: 147 CTAs).  The solve is FP64;
+// complex64 fields are widened as they are staged and rounded as they leave.
 // Systems are solved with N rows, N the smallest of 64, 128, 256, 512, 768
 // and 1024 that holds the grid's n (h.n): rows n .. N-1 are decoupled (their
 // factors g = 1, h = 0, right-hand sides zero, nothing copied in or out),
@@ -517,8 +518,8 @@ static cudaError_t adi_const_launch(const AdiHalf &h, const void *g, const void 
 // bytes each -- measured slower than per-thread copies: the copy engine's
 // per-request cost dominates at these sizes.)
 //
-// Compute: the CTA's systems form two groups (GS0 = ceil(G/2) and G - GS0
-// systems); a thread owns one chunk of M rows of every system of its group.
+// Compute: the CTA's systems form groups of S (two; one where a CTA holds just
+// two systems); a thread owns one chunk of M rows of every system of its group.
 // Each staged value is read from shared memory once and serves the three
 // stencils it enters, each factor-table entry serves all systems of the
 // group, and the sweeps run the group's independent recurrences side by
