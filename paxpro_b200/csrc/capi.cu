@@ -17,6 +17,7 @@
 #include <atomic>
 #include <cmath>
 #include <map>
+#include <memory>
 #include <tuple>
 #include <complex>
 #include <cstdio>
@@ -579,24 +580,31 @@ int cn_set_planes(pxp_solver_s *h, const double *delta, const double *beta, int 
   // nsteps * n doubles; per-step stride n.
   const unsigned n = h->nx;
   const size_t per = (size_t)n * nsteps;
-  std::vector<double> buf(4 * per);
+  std::unique_ptr<double[]> buf(new double[4 * per]);  // every entry is written below
+  auto put = [&](int block, int step, const double *src) {
+    double *dst = &buf[block * per + (size_t)step * n];
+    std::memcpy(dst, src, sizeof(double) * n);
+    long long beyond = 0;  // few media have any; a count over the row just copied vectorizes
+    for (unsigned i = 0; i < n; ++i) beyond += std::fabs(dst[i]) > pxp::kOpaque ? 1 : 0;
+    if (beyond > 0)
+      for (unsigned i = 0; i < n; ++i) dst[i] = pxp::opaque(dst[i]);
+  };
   for (int s = 0; s < nsteps; ++s) {
     const size_t src0 = (size_t)(two_planes_per_step ? 2 * s : s) * n;
     const size_t src1 = (size_t)(two_planes_per_step ? 2 * s + 1 : s) * n;
-    std::memcpy(&buf[0 * per + (size_t)s * n], delta + src0, sizeof(double) * n);
-    std::memcpy(&buf[1 * per + (size_t)s * n], beta + src0, sizeof(double) * n);
-    std::memcpy(&buf[2 * per + (size_t)s * n], delta + src1, sizeof(double) * n);
-    std::memcpy(&buf[3 * per + (size_t)s * n], beta + src1, sizeof(double) * n);
+    put(0, s, delta + src0);
+    put(1, s, beta + src0);
+    put(2, s, delta + src1);
+    put(3, s, beta + src1);
   }
-  for (double &v : buf) v = pxp::opaque(v);
   h->medium_ok = false;
   h->cn_const = h->cn_vacuum = false;
   cn_win_release(h, h->stream);
   free_dev(h->d_mat, h->stream);
   int rc;
-  if ((rc = alloc(h, (void **)&h->d_mat, sizeof(double) * buf.size(), "material planes")))
+  if ((rc = alloc(h, (void **)&h->d_mat, sizeof(double) * 4 * per, "material planes")))
     return rc;
-  if (int rc_ = h2d(h, h->d_mat, buf.data(), sizeof(double) * buf.size())) return rc_;
+  if (int rc_ = h2d(h, h->d_mat, buf.get(), sizeof(double) * 4 * per)) return rc_;
   h->mat_block = (long long)per;
   h->mat_stride = nsteps > 1 ? n : 0;
   h->mat_step0 = first_step;

@@ -14,8 +14,9 @@ enum Precision { kFP64 = 0, kFP32 = 1 };
 // A medium's delta or beta as the tridiagonal solves take it: opaque beyond
 // measure is opaque, and the squares of the matrix entries stay finite.  Values
 // stored on the host are limited there, planes where they are read.
+constexpr double kOpaque = 1e140;
 __host__ __device__ inline double opaque(double v) {
-  return v > 1e140 ? 1e140 : v < -1e140 ? -1e140 : v;
+  return v > kOpaque ? kOpaque : v < -kOpaque ? -kOpaque : v;
 }
 
 // Record the message pxp_last_error(NULL, ...) returns (capi.cu).
