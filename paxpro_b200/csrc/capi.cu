@@ -1284,7 +1284,10 @@ int sms_of_others(int device, int nj) {
 int cn_write_job(pxp_solver_s *h);
 
 // A CrankNicholson solver that steps before any material is set: its vacuum
-// tables.
+// tables, made when it gets its initial conditions, so that a first step under
+// stream capture finds them, or at a first step or admission that comes
+// otherwise.  (At creation most solvers would pay for tables that their material
+// replaces: 0.2 ms at 4096 rows.)
 int cn_vacuum_tables(pxp_solver_s *h) {
   if (!h->cn_vacuum || !cn_uses_const(h)) return PXP_OK;
   const std::vector<double> zeros(h->npts, 0.0);
@@ -1943,10 +1946,14 @@ static int download_field(pxp_solver_s *h, double *dst, const void *src, long lo
   return PXP_OK;
 }
 
-int pxp_set_initial_conditions(pxp_solver h, const double *field) {
-  if (h == nullptr || field == nullptr) return PXP_ERR_INVALID;
-  int rc = upload_field(h, h->d_field, field);
-  if (rc) return rc;
+// A field has been put in place: the handle can step.
+static int field_set(pxp_solver_s *h) {
+  if (h->cn_vacuum) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    PXP_TRY_CUDA(h, cudaStreamIsCapturing(h->stream, &cap));
+    if (cap == cudaStreamCaptureStatusNone)
+      if (int rc = cn_vacuum_tables(h)) return rc;
+  }
   h->current_step = 1;
   h->cn_win_count = 0;  // tables serve one pass through the medium
   h->ic_set = true;
@@ -1954,15 +1961,17 @@ int pxp_set_initial_conditions(pxp_solver h, const double *field) {
   return PXP_OK;
 }
 
+int pxp_set_initial_conditions(pxp_solver h, const double *field) {
+  if (h == nullptr || field == nullptr) return PXP_ERR_INVALID;
+  if (int rc = upload_field(h, h->d_field, field)) return rc;
+  return field_set(h);
+}
+
 int pxp_set_initial_conditions_device(pxp_solver h, const void *dfield) {
   if (h == nullptr || dfield == nullptr) return PXP_ERR_INVALID;
   PXP_TRY_CUDA(h, cudaMemcpyAsync(h->d_field, dfield, h->csize * h->npts,
                                   cudaMemcpyDeviceToDevice, h->stream));
-  h->current_step = 1;
-  h->cn_win_count = 0;
-  h->ic_set = true;
-  set_busy(h, true);
-  return PXP_OK;
+  return field_set(h);
 }
 
 int pxp_step(pxp_solver h, int nsteps) {

@@ -4,14 +4,15 @@
 // launch is only counted.  fake_fail_allocations(k) makes the k-th
 // cudaMallocAsync from then on fail, and those after it (0: none);
 // fake_launches() is the number of launches so far, fake_last_grid() the CTAs of
-// the last one, fake_live() the cudaMallocAsync allocations not yet freed;
+// the last one, fake_copies() that of cudaMemcpyAsync calls, fake_live() the
+// cudaMallocAsync allocations not yet freed;
 // fake_capturing(1) has streams report that they are being captured.
 #include <cuda_runtime_api.h>
 
 #include <cstdlib>
 #include <cstring>
 
-static long g_launches = 0, g_fail_at = 0, g_allocs = 0, g_grid = 0, g_live = 0;
+static long g_launches = 0, g_fail_at = 0, g_allocs = 0, g_grid = 0, g_live = 0, g_copies = 0;
 static int g_capturing = 0;
 
 extern "C" {
@@ -23,6 +24,7 @@ void fake_fail_allocations(long k) {
 long fake_launches() { return g_launches; }
 long fake_last_grid() { return g_grid; }
 long fake_live() { return g_live; }
+long fake_copies() { return g_copies; }
 void fake_capturing(int on) { g_capturing = on; }
 
 static cudaError_t give(void **p, size_t n) {
@@ -65,6 +67,7 @@ cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) {
   return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) {
+  ++g_copies;
   std::memcpy(d, s, n);
   return cudaSuccess;
 }

@@ -136,3 +136,18 @@ def test_large_batches_go_step_by_step():
                 j.close()
             b.close()
     """)
+
+
+def test_a_first_step_without_a_material_can_be_captured():
+    """Nothing is allocated or copied by it."""
+    fake_cuda.run("""
+        for n in (100, 4096):
+            s = pxp.Solver(spec(pxp.CRANK_NICHOLSON, n))
+            s.set_initial_conditions(np.ones(n, dtype=np.complex128))
+            held, copies = fake.fake_live(), fake.fake_copies()
+            fake.fake_capturing(1)
+            s.step(3)
+            fake.fake_capturing(0)
+            assert (fake.fake_live(), fake.fake_copies()) == (held, copies)
+            s.close()
+    """)
