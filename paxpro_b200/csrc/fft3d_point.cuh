@@ -149,8 +149,9 @@ __device__ __forceinline__ typename Cx<R>::T refract3(const Fft3dPass &q, typena
   }
   // (u * t) / (n*n): when n*n is a power of two, multiplying by its exact
   // reciprocal rounds identically to the division; other sizes pass
-  // inv_norm = 0 and divide (div_by)
-  u = inv_norm != 0.0 ? cx_scale_rn(u, inv_norm) : cx_div_by(u, Divisor{q.norm, q.inv_norm});
+  // inv_norm = 0 and divide
+  const Divisor nn{q.norm, q.inv_norm};
+  u = inv_norm != 0.0 ? cx_scale_rn(u, inv_norm) : mk(div_by_tested(u.x, nn), div_by_tested(u.y, nn));
   if (q.thick_y > 0) {
     if (iy < q.thick_y) u = cx_scale_rn(u, exp(-(double)(q.thick_y - iy - 1) * q.inv_damp_y));
     if (q.n - 1 - iy < q.thick_y)

@@ -27,7 +27,7 @@ __device__ unsigned long long ulps(double a, double b) {
 
 // [0] largest difference of rcp_newton over its range; [1] values wrong at its ends;
 // [2] div_by: normal results that differ; [3] largest difference of subnormal
-// ones; [4] special values wrong
+// ones; [4] special values wrong, or the two forms of the division differ
 __global__ void check(unsigned long long *out) {
   const unsigned long long id = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
   // every exponent whose reciprocal is normal: 2^-1022 <= m <= 2^1022
@@ -50,6 +50,7 @@ __global__ void check(unsigned long long *out) {
     for (int e = 1; e < 2047; e += 7) {
       const double a = draw((id * 64 + k) * 4096 + e, e, true);
       const double got = div_by(a, d), want = __ddiv_rn(a, s);
+      if (ulps(got, div_by_tested(a, d))) atomicAdd(out + 4, 1ull);
       if (fabs(want) >= tiny) {
         if (ulps(got, want)) atomicAdd(out + 2, 1ull);
       } else {
@@ -60,9 +61,10 @@ __global__ void check(unsigned long long *out) {
     atomicMax(out + 3, ulps(div_by(z, d), __ddiv_rn(z, s)));
     const double special[] = {0.0, -0.0, inf, -inf, huge, -huge, sub, -sub, tiny, -tiny};
     for (double a : special)
-      if (__double_as_longlong(div_by(a, d)) != __double_as_longlong(__ddiv_rn(a, s)))
+      if (ulps(div_by(a, d), __ddiv_rn(a, s)) || ulps(div_by_tested(a, d), __ddiv_rn(a, s)))
         atomicAdd(out + 4, 1ull);
-    if (div_by(nan, d) == div_by(nan, d)) atomicAdd(out + 4, 1ull);
+    if (div_by(nan, d) == div_by(nan, d) || div_by_tested(nan, d) == div_by_tested(nan, d))
+      atomicAdd(out + 4, 1ull);
   }
 }
 
